@@ -136,7 +136,11 @@ struct isspa_engine {
     float *g_raw = nullptr;
     int *nbp = nullptr;
     // adjoint buffers (allocated on first use)
-    int *point_win = nullptr, *adj_off = nullptr, *adj_atoms = nullptr;
+    int4 *adj_items = nullptr;  // force work items of the tiles that hold a restrained atom
+    int2 *adj_chunks = nullptr;
+    int n_adj_items = 0;
+    int *adj_off = nullptr, *adj_atoms = nullptr;
+    double *adj_s = nullptr, *axis = nullptr;
     double *cvec = nullptr, *lam = nullptr, *grads = nullptr;
     int n_adj_cap = 0;
     double *com = nullptr, *cv = nullptr;
@@ -1425,16 +1429,40 @@ int isspa_adjoint_mean_force(isspa_engine *e, int n_frames, const float *frames,
             e->raw_e = e->alloc<float4>(P);
             e->raw_e0 = e->alloc<float4>(P);
         }
-        if (!e->point_win) {
-            std::vector<int> pw(P);
-            for (int w = 0; w < W; ++w)
-                for (long long p = 0; p < (long long)e->win_h[w].n_atoms * e->n_mc; ++p) pw[e->win_h[w].point_off + p] = w;
-            e->point_win = e->upload(pw);
+        if (!e->cvec) {
             e->cvec = e->alloc<double>(3 * (size_t)N);
             e->lam = e->alloc<double>(P);
             e->grads = e->alloc<double>((size_t)W * per_w);
             e->adj_off = e->alloc<int>(W + 1);
             e->adj_atoms = e->alloc<int>(std::max<size_t>(1, e->bias_h.size()));
+            e->adj_s = e->alloc<double>(std::max<size_t>(1, e->bias_h.size()));
+            e->axis = e->alloc<double>(3 * (size_t)W);
+        }
+        // J weighs restrained atoms only: the IS-SPA force pass runs on the 128-atom
+        // tiles that hold one (16 windows x 550 atoms: one tile of five), in
+        // chunks of 128 points so that those tiles alone fill the GPU
+        if (!e->adj_items) {
+            std::vector<char> biased(N, 0);
+            for (const int2 &b : e->bias_h) biased[b.x] = 1;
+            std::vector<int4> items;
+            std::vector<int2> chunks;
+            for (int w = 0; w < W; ++w) {
+                const WinDev &d = e->win_h[w];
+                std::vector<int> tiles;
+                for (int t = 0; t < d.n_atoms; t += 128) {
+                    const auto first = biased.begin() + d.atom_off + t, last = first + std::min(128, d.n_atoms - t);
+                    if (std::find(first, last, 1) != last) tiles.push_back(t);
+                }
+                const long long np = (long long)d.n_atoms * e->n_mc;
+                for (long long p = 0; !tiles.empty() && p < np; p += 128) {
+                    for (int t : tiles)
+                        items.push_back(make_int4(w, d.atom_off + t, std::min(128, d.n_atoms - t), (int)chunks.size()));
+                    chunks.push_back(make_int2((int)(d.point_off + p), (int)std::min<long long>(128, np - p)));
+                }
+            }
+            e->adj_chunks = e->upload(chunks);
+            e->adj_items = e->upload(items);
+            e->n_adj_items = (int)items.size();
         }
         // Every copy below is ordered on the engine's (non-blocking) stream: a
         // legacy-stream cudaMemcpy does not wait for the previous frame's
@@ -1453,6 +1481,7 @@ int isspa_adjoint_mean_force(isspa_engine *e, int n_frames, const float *frames,
             // weights c_i = +-n/2 on the two restraint groups of each window
             std::fill(cvec.begin(), cvec.end(), 0.0);
             std::vector<int> off(W + 1, 0), atoms;
+            std::vector<double> atom_s, axis(3 * (size_t)W, 0.0);
             for (int w = 0; w < W; ++w) {
                 off[w] = (int)atoms.size();
                 const WinDev &d = e->win_h[w];
@@ -1474,24 +1503,38 @@ int isspa_adjoint_mean_force(isspa_engine *e, int n_frames, const float *frames,
                     nn += v * v;
                 }
                 nn = std::sqrt(nn);
+                for (int k = 0; k < 3; ++k) axis[3 * (size_t)w + k] = n[k] / nn;
                 for (int b = 0; b < d.n_bias; ++b) {
                     const int2 bl = e->bias_h[d.bias_off + b];
                     const double sgn = bl.y == 0 ? 0.5 : -0.5;
                     for (int k = 0; k < 3; ++k) cvec[3 * (size_t)bl.x + k] += sgn * n[k] / nn;
-                    if (std::find(atoms.begin() + off[w], atoms.end(), bl.x) == atoms.end()) atoms.push_back(bl.x);
+                    const size_t at = (size_t)(std::find(atoms.begin() + off[w], atoms.end(), bl.x) - atoms.begin());
+                    if (at == atoms.size()) {
+                        atoms.push_back(bl.x);
+                        atom_s.push_back(0.0);
+                    }
+                    atom_s[at] += sgn;
                 }
             }
             off[W] = (int)atoms.size();
             ck(cudaMemcpyAsync(e->cvec, cvec.data(), sizeof(double) * cvec.size(), cudaMemcpyHostToDevice, e->stream));
             ck(cudaMemcpyAsync(e->adj_off, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice, e->stream));
-            if (!atoms.empty())
+            ck(cudaMemcpyAsync(e->axis, axis.data(), sizeof(double) * axis.size(), cudaMemcpyHostToDevice, e->stream));
+            if (!atoms.empty()) {
                 ck(cudaMemcpyAsync(e->adj_atoms, atoms.data(), sizeof(int) * atoms.size(), cudaMemcpyHostToDevice,
                                    e->stream));
+                ck(cudaMemcpyAsync(e->adj_s, atom_s.data(), sizeof(double) * atoms.size(), cudaMemcpyHostToDevice,
+                                   e->stream));
+            }
             // the value: every non-restraint force of the frame, projected
             ck(cudaMemsetAsync(e->facc, 0, 3 * sizeof(unsigned long long) * N, e->stream));
             launch_bonded(e->bonded_args(1, 1, 1), e->stream);
             launch_field(e->field_args(), e->field_split, true, e->stream);
-            launch_force(e->force_args(), e->stream);
+            ForceArgs fa = e->force_args();
+            fa.items = e->adj_items;
+            fa.chunks = e->adj_chunks;
+            fa.n_items = e->n_adj_items;
+            launch_force(fa, e->stream);
             launch_nonbond(e->nonbond_args(), e->stream);
             ck(cudaGetLastError());
             ck(cudaMemcpyAsync(acc.data(), e->facc, sizeof(long long) * acc.size(), cudaMemcpyDeviceToHost, e->stream));
@@ -1507,14 +1550,17 @@ int isspa_adjoint_mean_force(isspa_engine *e, int n_frames, const float *frames,
             a.atype = e->atype;
             a.win = e->win;
             a.atom_win = e->atom_win;
-            a.n_points = P;
-            a.point_win = e->point_win;
+            a.n_windows = W;
+            a.stage = adjoint_stage(e->max_window_atoms());
+            a.tiles_max = (int)(((long long)e->max_window_atoms() * e->n_mc + adjoint_point_tile() - 1) / adjoint_point_tile());
             a.raw_e = e->raw_e;
             a.raw_e0 = e->raw_e0;
             a.q0 = e->pts.q0;
             a.adj_off = e->adj_off;
             a.adj_atoms = e->adj_atoms;
             a.n_adj = (int)atoms.size();
+            a.adj_s = e->adj_s;
+            a.axis = e->axis;
             a.cvec = e->cvec;
             a.rmax = e->rmax;
             a.vtot = e->vtot;

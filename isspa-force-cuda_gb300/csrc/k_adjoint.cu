@@ -12,150 +12,275 @@
 //   scaled 1-4 LJ (dih_force_cuda.cu:70-74), which are linear in A and B.
 // MC points are the field pass's (regenerated from the Philox counters of the
 // frame's step); gradients accumulate in FP64 per window.
+//
+// GB300's FP64 pipe takes a warp instruction every 16 cycles per SM (an FP32
+// one: a quarter of a cycle), whether one lane or 32 are active, so the points
+// and density kernels work in double-float on the FP32 pipe and leave FP64 to
+// the sums.  16 windows x 550 atoms, nMC 50, per launch: points 6.76 ms in FP64,
+// 0.30 in double-float; density 12.0 ms, 2.4 with the double-float body, 0.91
+// once the warp reconverges after each lane's own atoms, 0.81 with one FP32 test
+// per atom and point; pairs 0.88 ms with a thread per atom, 0.07 with a warp.
+// The error against 64-bit references is the FP32 fields' and coordinates'
+// either way (6e-6 of dJ/dT_g at those sizes, before and after).
+#include <algorithm>
 #include <cuda_runtime.h>
 
+#include "dfloat.cuh"
 #include "kernels.h"
 
 namespace isspa {
 namespace {
 
-__device__ __forceinline__ void langevin_d(float x, double &p1, double &p2, double &p3) {
-    // backward continued fraction of i_l/i_(l-1) (all terms positive)
-    if (x < 5.0f) {
-        double r = 0.0, r2 = 0.0, r3 = 0.0;
-        for (int l = 24; l >= 1; --l) {
-            r = (double)x / ((double)(2 * l + 1) + (double)x * r);
-            if (l == 3) r3 = r;
-            if (l == 2) r2 = r;
+constexpr int kAdjThreads = 128;
+constexpr int kAdjStage = 1024;  // most atoms staged at a time (32 groups of 32)
+
+__device__ __forceinline__ DF df_const(double c) { return DF{(float)c, (float)(c - (double)(float)c)}; }  // folded
+
+// <P1>, <P2>, <P3> of a Langevin dipole in a field x.  Below 5 the backward
+// continued fraction r_l = x / (2l+1 + x r_(l+1)) is carried as numerators and
+// denominators, A_l = x B_(l+1), B_l = (2l+1) B_(l+1) + x A_(l+1) (all terms
+// positive), so that <P_m> = r_1 ... r_m = x^m B_(m+1) / B_1 takes one division
+// instead of one per level; 18 levels leave 1e-19 at x = 5.  Above, the closed
+// forms with coth x = (1 + q) / (1 - q), q = exp(-2x).
+__device__ __forceinline__ void langevin_df(DF x, DF &p1, DF &p2, DF &p3) {
+    if (x.hi < 5.0f) {
+        DF A{0.f, 0.f}, B{1.f, 0.f}, b2 = B, b3 = B, b4 = B;
+#pragma unroll 3
+        for (int l = 18; l >= 1; --l) {
+            const DF nb = df_add(df_mulf(B, (float)(2 * l + 1)), df_mul(x, A));
+            A = df_mul(x, B);
+            B = nb;
+            if (l == 4) b4 = B;
+            if (l == 3) b3 = B;
+            if (l == 2) b2 = B;
         }
-        p1 = r;
-        p2 = r * r2;
-        p3 = r * r2 * r3;
+        p1 = df_div(A, B);  // A_1 = x B_2
+        const DF x2 = df_mul(x, x);
+        p2 = df_div(df_mul(x2, b3), B);
+        p3 = df_div(df_mul(df_mul(x2, x), b4), B);
     } else {
-        const double X = x, c = 1.0 / tanh(X), ix = 1.0 / X;
-        p1 = c - ix;
-        p2 = 1.0 + 3.0 * ix * ix - 3.0 * c * ix;
-        p3 = (1.0 + 15.0 * ix * ix) * c - 6.0 * ix - 15.0 * ix * ix * ix;
+        const DF q = df_from(exp(-2.0 * df_double(x)));
+        const DF c = df_div(df_addf(q, 1.0f), df_addf(df_neg(q), 1.0f));
+        const DF ix = df_div(DF{1.f, 0.f}, x), ix2 = df_mul(ix, ix), cx = df_mul(c, ix);
+        p1 = df_add(c, df_neg(ix));
+        p2 = df_addf(df_mulf(df_add(ix2, df_neg(cx)), 3.0f), 1.0f);
+        p3 = df_add(df_add(c, df_mulf(df_mul(ix2, df_add(c, df_neg(ix))), 15.0f)), df_mulf(ix, -6.0f));
     }
 }
 
-__global__ void adjoint_points_kernel(AdjointArgs a) {
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= a.n_points) return;
-    const int w = a.point_win[p];
+// hi + lo in FP64 with one FP64 instruction: a float widens to a double with
+// integer operations (exponent rebiased by 896, mantissa moved up by 29 bits;
+// zeros and infinities / NaN keep their exponents).
+__device__ __forceinline__ double widen(float v) {
+    const unsigned u = __float_as_uint(v), m = u & 0x7fffffffu;
+    unsigned e = (m >> 3) + 0x38000000u;
+    e = m >= 0x7f800000u ? (m >> 3) | 0x7ff00000u : e;
+    e = m < 0x00800000u ? 0u : e;
+    return __hiloint2double((int)((u & 0x80000000u) | e), (int)(m < 0x00800000u ? 0u : u << 29));
+}
+__device__ __forceinline__ double df_sum(DF a) { return widen(a.hi) + widen(a.lo); }
+
+// A block's window and point tile: blocks are window-major, tiles_max per
+// window; false when the window has no restraint or no such tile.
+__device__ __forceinline__ bool adj_tile(const AdjointArgs &a, int &w, long long &p, bool &valid) {
+    w = blockIdx.x / a.tiles_max;
+    const long long q = (long long)(blockIdx.x % a.tiles_max) * kAdjThreads;
+    const WinDev &W = a.win[w];
+    const long long n = (long long)W.n_atoms * a.n_mc;
+    if (!W.us_on || q >= n) return false;
+    valid = q + threadIdx.x < n;
+    p = W.point_off + q + (valid ? threadIdx.x : 0);
+    return true;
+}
+
+// One weighted atom, staged for a block of points: weights c_i = s_i n with n
+// the window's COM axis.
+struct AdjAtom {
+    float4 x;
+    float cs_hi, cs_lo;  // -vtot s_i
+    float rm2;
+    int frow;
+};
+
+// lambda_p and dJ/dT_f of one point per thread.  Per pair, with e the unit
+// field, w = e.r, g = w / r^2 and the per-unit-density amplitudes a_l:
+//   n . G = -q_i vtot r^-3 [ (n.r) 3 X / r^2 - (n.e) (Y + a1) ] - vtot (n.r) T_f / r,
+//   X = g (w (2.5 a2 + 35/6 a3 g) - 2.5 a3) + a1 w - a2/2,
+//   Y = (7.5 a3 g + 3 a2) g - 1.5 a3 / r^2
+// (the multipole terms of src/isspa_force_cuda.cu:274-289 projected on n).
+__global__ void __launch_bounds__(kAdjThreads) adjoint_points_kernel(AdjointArgs a) {
+    __shared__ AdjAtom s_at[kAdjThreads];
+    int w;
+    long long p;
+    bool valid;
+    if (!adj_tile(a, w, p, valid)) return;
     const WinDev W = a.win[w];
-    if (!W.us_on) return;
     const float4 raw = a.raw_e[p], raw0 = a.raw_e0[p];
     const float4 P = a.q0[p];
-    const int n = (int)raw0.w;
-    const double inv_n = 1.0 / (double)n, sp = (double)raw.w * inv_n;
-    const double mag = sqrt((double)raw.x * raw.x + (double)raw.y * raw.y + (double)raw.z * raw.z);
-    double p1, p2, p3;
-    langevin_d((float)mag, p1, p2, p3);
-    const double eh[3] = {mag > 0 ? raw.x / mag : 0.0, mag > 0 ? raw.y / mag : 0.0, mag > 0 ? raw.z / mag : 0.0};
+    const DF sp = df_div(DF{raw.w, 0.f}, DF{(float)(int)raw0.w, 0.f});
+    const DF e2 = df_norm2(raw.x, raw.y, raw.z);
+    const DF im = e2.hi > 0.0f ? df_rsqrt(e2) : DF{0.f, 0.f};
+    DF A1, a2, a3;
+    langevin_df(df_mul(e2, im), A1, a2, a3);
+    A1 = df_mulf(A1, kP0);
+    a2 = df_mulf(a2, kQ0);
+    a3 = df_mulf(a3, kO0);
+    const DF ex = df_mulf(im, raw.x), ey = df_mulf(im, raw.y), ez = df_mulf(im, raw.z);
+    const double *n3 = a.axis + 3 * w;
+    const DF nx = df_from(n3[0]), ny = df_from(n3[1]), nz = df_from(n3[2]);
+    const DF en = df_add(df_add(df_mul(ex, nx), df_mul(ey, ny)), df_mul(ez, nz));
+    const DF c0 = df_mulf(a2, -0.5f), kx = df_mulf(a2, 2.5f), ky = df_mul(a3, df_const(35.0 / 6.0)),
+             k25 = df_mulf(a3, -2.5f), y1 = df_mulf(a3, 7.5f), y0 = df_mulf(a2, 3.0f), u15 = df_mulf(a3, -1.5f);
+    const DF f_inv = df_div(DF{1.f, 0.f}, DF{a.f_dr, 0.f});
     const float L = W.box, h = W.hbox;
-    double lam = 0.0;
-    for (int k = a.adj_off[w]; k < a.adj_off[w + 1]; ++k) {
-        const int i = a.adj_atoms[k];
-        const double c0 = a.cvec[3 * i], c1 = a.cvec[3 * i + 1], c2 = a.cvec[3 * i + 2];
-        const float4 xi = a.pos[i];
-        const int it = a.atype[i].y;
-        const float rm = __ldg(a.rmax + it);
-        const double vt = __ldg(a.vtot + it), qi = xi.w;
-        const float rx = mimg(P.x - xi.x, L, h), ry = mimg(P.y - xi.y, L, h), rz = mimg(P.z - xi.z, L, h);
-        const float d2 = dist2f(rx, ry, rz);
-        const double r[3] = {rx, ry, rz};
-        const double dd2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2], dd = sqrt(dd2);
-        const double Rz = (eh[0] * r[0] + eh[1] * r[1] + eh[2] * r[2]) / dd;
-        const double dp1 = 3.0 * Rz, dp2 = 7.5 * Rz * Rz - 1.5, dp3 = (17.5 * Rz * Rz - 7.5) * Rz;
-        const double t1 = (double)kP0 * p1 / (dd2 * dd), t2 = (double)kQ0 * p2 / (dd2 * dd2),
-                     t3 = (double)kO0 * p3 / (dd2 * dd2 * dd);
-        double G = 0.0;
-        const double cc[3] = {c0, c1, c2};
-        for (int d = 0; d < 3; ++d) {
-            const double mu = t1 * (r[d] * dp1 / dd - eh[d]) + t2 * (r[d] * dp2 / dd - dp1 * eh[d]) +
-                              t3 * (r[d] * dp3 / dd - dp2 * eh[d]);
-            G += cc[d] * (-qi * vt * mu);
+    DF lam{0.f, 0.f};
+    const int k1 = a.adj_off[w + 1];
+    for (int k0 = a.adj_off[w]; k0 < k1; k0 += kAdjThreads) {
+        const int kn = min(kAdjThreads, k1 - k0);
+        __syncthreads();
+        if (threadIdx.x < kn) {
+            const int i = a.adj_atoms[k0 + threadIdx.x];
+            const int it = a.atype[i].y;
+            const float rm = __ldg(a.rmax + it);
+            const DF cs = df_from(-(double)__ldg(a.vtot + it) * a.adj_s[k0 + threadIdx.x]);
+            s_at[threadIdx.x] = AdjAtom{a.pos[i], cs.hi, cs.lo, __fmul_rn(rm, rm), it * a.n_f};
         }
-        if (d2 <= __fmul_rn(rm, rm)) {
-            const float dist = __fsqrt_rn(d2);
-            const int bin = (int)__fmaf_rn(__fsub_rn(dist, a.f_r0), a.f_inv, 0.5f);
-            if (bin >= 0 && bin < a.n_f) {
-                const double fr = (dd - ((double)a.f_r0 + bin * (double)a.f_dr)) / a.f_dr;
-                const long long fi = (long long)it * a.n_f + bin;
-                const float2 tv = __ldg(a.ftab + fi);
-                const double tab = tv.x * (1.0 - fr) + tv.y * fr;
-                const double cr = -vt * (c0 * r[0] + c1 * r[1] + c2 * r[2]) / dd;
-                G += cr * tab;
-                double *df = a.dJ_df + (long long)w * a.n_ftab;
-                atomicAdd(df + fi, cr * sp * (1.0 - fr));
-                if (fi + 1 < a.n_ftab) atomicAdd(df + fi + 1, cr * sp * fr);
-            }
-        }
-        lam += G;
-    }
-    a.lam[p] = lam;
-}
-
-__global__ void adjoint_density_kernel(AdjointArgs a) {
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= a.n_points) return;
-    const int w = a.point_win[p];
-    const WinDev W = a.win[w];
-    if (!W.us_on) return;
-    const double lam = a.lam[p];
-    if (lam == 0.0) return;
-    const float4 P = a.q0[p];
-    const int n = (int)a.raw_e0[p].w;
-    const double dJdw = lam / (double)n;
-    const int owner = W.atom_off + (int)((p - W.point_off) / a.n_mc);
-    const float rm = __ldg(a.rmax + a.atype[owner].y);
-    const float rm2 = __fmul_rn(rm, rm);
-    const float L = W.box, h = W.hbox;
-    int zeros = 0, forced = 0;
-    double prod = 1.0;
-    double *dg = a.dJ_dg + (long long)w * a.n_gtab;
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int j = W.atom_off; j < W.atom_off + W.n_atoms; ++j) {
-            const float4 xj = a.pos[j];
-            const float rx = mimg(P.x - xj.x, L, h), ry = mimg(P.y - xj.y, L, h), rz = mimg(P.z - xj.z, L, h);
-            const float d2 = dist2f(rx, ry, rz);
-            if (!(d2 <= rm2)) continue;
-            const float dist = __fsqrt_rn(d2);
-            const int bin = (int)__fmul_rn(__fsub_rn(dist, a.g_r0), a.g_inv);
-            if (bin < 0) {
-                forced = 1;
-                continue;
-            }
-            if (bin >= a.n_g - 1) continue;
-            const double dd = sqrt((double)rx * rx + (double)ry * ry + (double)rz * rz);
-            const double fr = (dd - ((double)a.g_r0 + bin * (double)a.g_dr)) / a.g_dr;
-            const long long gi = (long long)a.atype[j].y * a.n_g + bin;
-            const double g0 = a.g_table[gi], g1 = gi + 1 < a.n_gtab ? a.g_table[gi + 1] : 0.0;
-            const double g = g0 * (1.0 - fr) + g1 * fr;
-            if (pass == 0) {
-                if (g == 0.0) ++zeros;
-                else prod *= g;
-            } else {
-                double others;
-                if (forced || zeros >= 2) others = 0.0;
-                else if (zeros == 1) others = g == 0.0 ? prod : 0.0;
-                else others = prod / g;
-                const double d = dJdw * others;
-                if (d != 0.0) {
-                    atomicAdd(dg + gi, d * (1.0 - fr));
-                    if (gi + 1 < a.n_gtab) atomicAdd(dg + gi + 1, d * fr);
+        __syncthreads();
+        for (int k = 0; k < kn; ++k) {
+            const AdjAtom at = s_at[k];
+            const float rx = mimg(P.x - at.x.x, L, h), ry = mimg(P.y - at.x.y, L, h), rz = mimg(P.z - at.x.z, L, h);
+            const DF d2 = df_norm2(rx, ry, rz);
+            const DF ri = df_rsqrt(d2), ri2 = df_mul(ri, ri), ri3 = df_mul(ri2, ri);
+            const DF er = df_add(df_add(df_mulf(ex, rx), df_mulf(ey, ry)), df_mulf(ez, rz));
+            const DF nr = df_add(df_add(df_mulf(nx, rx), df_mulf(ny, ry)), df_mulf(nz, rz));
+            const DF g = df_mul(er, ri2);
+            const DF X = df_add(df_fma(g, df_fma(er, df_fma(ky, g, kx), k25), c0), df_mul(A1, er));
+            const DF Z = df_mulf(df_mul(ri2, X), 3.0f);
+            const DF Y = df_add(df_add(df_mul(df_fma(y1, g, y0), g), df_mul(u15, ri2)), A1);
+            DF G = df_mulf(df_mul(ri3, df_add(df_mul(nr, Z), df_neg(df_mul(en, Y)))), at.x.w);
+            const DF cs{at.cs_hi, at.cs_lo};
+            const float d2f = dist2f(rx, ry, rz);
+            if (valid && d2f <= at.rm2) {
+                const int bin = (int)__fmaf_rn(__fsub_rn(__fsqrt_rn(d2f), a.f_r0), a.f_inv, 0.5f);
+                if (bin >= 0 && bin < a.n_f) {
+                    const DF fr = df_table_frac(df_mul(d2, ri), a.f_r0, f_inv, bin);
+                    const long long fi = at.frow + bin;
+                    const float2 tv = __ldg(a.ftab + fi);
+                    const DF tab = df_lerp(tv.x, tv.y, fr);
+                    const DF cr = df_mul(nr, ri);
+                    G = df_fma(cr, tab, G);
+                    const DF c = df_mul(df_mul(cr, cs), sp), cf = df_mul(c, fr);
+                    double *df = a.dJ_df + (long long)w * a.n_ftab;
+                    atomicAdd(df + fi, df_sum(df_add(c, df_neg(cf))));
+                    if (fi + 1 < a.n_ftab) atomicAdd(df + fi + 1, df_sum(cf));
                 }
             }
+            lam = df_fma(G, cs, lam);
         }
+    }
+    if (valid) a.lam[p] = df_double(lam);
+}
+
+// dJ/dT_g of one point per thread, in two sweeps over the point's in-range
+// atoms: the density product, then every factor's share lambda/n * prod / g.
+// The window's atoms are tested once in FP32 (once per sweep for windows beyond
+// one stage), 32 to a mask in shared memory, and each lane then walks its own
+// masks: the lanes' in-range atoms differ (a quarter of the atoms are inside
+// rmax of some lane of the warp at 550 atoms, 6 % of one lane's), so the
+// double-float work runs as often as the busiest lane has atoms instead of once
+// per atom that any lane has.  Strided groups spread a chain's atoms over masks.
+__global__ void __launch_bounds__(kAdjThreads, 10) adjoint_density_kernel(AdjointArgs a) {
+    extern __shared__ float4 s_x[];  // [stage] atoms, then [stage / 32][kAdjThreads] masks
+    const int stage = a.stage;
+    auto s_mask = reinterpret_cast<unsigned(*)[kAdjThreads]>(s_x + stage);
+    int w;
+    long long p;
+    bool valid;
+    if (!adj_tile(a, w, p, valid)) return;
+    const WinDev W = a.win[w];
+    const double lam = a.lam[p];
+    const float4 P = a.q0[p];
+    const int n = (int)a.raw_e0[p].w;
+    const DF dJdw = df_div(df_from(lam), DF{(float)n, 0.f});
+    const int owner = W.atom_off + (int)((p - W.point_off) / a.n_mc);
+    const float rm = __ldg(a.rmax + a.atype[owner].y);
+    // a lane with nothing to add takes no atom as in range
+    const float rm2 = valid && lam != 0.0 ? __fmul_rn(rm, rm) : -1.0f;
+    const float L = W.box, h = W.hbox;
+    const DF g_inv = df_div(DF{1.f, 0.f}, DF{a.g_dr, 0.f});
+    int zeros = 0;
+    bool forced = false;
+    DF prod{1.0f, 0.0f};
+    double *dg = a.dJ_dg + (long long)w * a.n_gtab;
+    const int N = W.n_atoms, t = threadIdx.x;
+    for (int pass = 0; pass < 2; ++pass) {
+        for (int j0 = 0; j0 < N; j0 += stage) {
+            const int jn = min(stage, N - j0);
+            const int nq = (jn + 31) >> 5;  // groups: atoms q, q + nq, q + 2 nq, ...
+            if (pass == 0 || N > stage) {
+                __syncthreads();
+                for (int i = t; i < jn; i += kAdjThreads) {
+                    float4 x = a.pos[W.atom_off + j0 + i];
+                    x.w = __int_as_float(a.atype[W.atom_off + j0 + i].y * a.n_g);
+                    s_x[i] = x;
+                }
+                __syncthreads();
+                for (int q = 0; q < nq; ++q) {
+                    unsigned mask = 0u, bit = 1u;
+#pragma unroll 4
+                    for (int k = q; k < jn; k += nq, bit <<= 1) {
+                        const float4 xj = s_x[k];
+                        const float d2 = dist2f(mimg(P.x - xj.x, L, h), mimg(P.y - xj.y, L, h), mimg(P.z - xj.z, L, h));
+                        if (d2 <= rm2) mask |= bit;
+                    }
+                    s_mask[q][t] = mask;  // read back by this thread only
+                }
+            }
+            int q = 0;
+            unsigned mask = s_mask[0][t];
+            for (;;) {
+                while (mask == 0u && ++q < nq) mask = s_mask[q][t];
+                if (mask == 0u) break;
+                const int k = q + (__ffs(mask) - 1) * nq;
+                mask &= mask - 1;
+                const float4 xj = s_x[k];
+                const float rx = mimg(P.x - xj.x, L, h), ry = mimg(P.y - xj.y, L, h), rz = mimg(P.z - xj.z, L, h);
+                const int bin = (int)__fmul_rn(__fsub_rn(__fsqrt_rn(dist2f(rx, ry, rz)), a.g_r0), a.g_inv);
+                forced |= bin < 0;
+                if (bin >= 0 && bin < a.n_g - 1) {
+                    const DF fr = df_table_frac(df_root(df_norm2(rx, ry, rz)), a.g_r0, g_inv, bin);
+                    const int gi = __float_as_int(xj.w) + bin;
+                    const bool next = gi + 1 < a.n_gtab;
+                    const float g0 = __ldg(a.g_table + gi), g1 = next ? __ldg(a.g_table + gi + 1) : 0.0f;
+                    const DF g = df_lerp(g0, g1, fr);
+                    if (pass == 0) {
+                        if (g.hi == 0.0f) ++zeros;
+                        else prod = df_mul(prod, g);
+                    } else if (!forced && (zeros == 0 || (zeros == 1 && g.hi == 0.0f))) {
+                        // (of zero factors only a single one's own share survives)
+                        const DF d = df_mul(dJdw, zeros ? prod : df_div(prod, g));
+                        if (d.hi != 0.0f) {
+                            const DF df = df_mul(d, fr);
+                            atomicAdd(dg + gi, df_sum(df_add(d, df_neg(df))));
+                            if (next) atomicAdd(dg + gi + 1, df_sum(df));
+                        }
+                    }
+                }
+            }
+            __syncwarp();  // the lanes leave the loop above at different times
+        }
+        // the second sweep has nothing to do for a lane whose every share is zero
+        if (forced || zeros >= 2)
+            for (int q = 0; N <= stage && q < (N + 31) >> 5; ++q) s_mask[q][t] = 0u;
+        __syncwarp();
     }
 }
 
-// Nonbond LJ coefficient adjoint for every weighted atom i (thread) against
+// Nonbond LJ coefficient adjoint of every weighted atom (one warp each) against
 // all atoms of its window; exclusions as the nonbond kernel.
-__global__ void adjoint_pairs_kernel(AdjointArgs a) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.n_adj) return;
+__global__ void __launch_bounds__(kAdjThreads) adjoint_pairs_kernel(AdjointArgs a) {
+    const int k = (blockIdx.x * kAdjThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (k >= a.n_adj) return;  // warp-uniform
     const int i = a.adj_atoms[k];
     const int w = a.atom_win[i];
     const WinDev W = a.win[w];
@@ -163,22 +288,25 @@ __global__ void adjoint_pairs_kernel(AdjointArgs a) {
     const float4 xi = a.pos[i];
     const int ti = a.atype[i].x;
     const float L = W.box, h = W.hbox;
-    int cur = a.excl_start[i];
-    const int end = a.excl_start[i + 1];
+    const int e0 = a.excl_start[i], e1 = a.excl_start[i + 1];
     double *dA = a.dJ_dA + (long long)w * a.n_ljtab, *dB = a.dJ_dB + (long long)w * a.n_ljtab;
-    for (int j = W.atom_off; j < W.atom_off + W.n_atoms; ++j) {
-        bool ex = false;
-        while (cur < end && a.excl[cur] < j) ++cur;
-        if (cur < end && a.excl[cur] == j) ex = true;
-        if (j == i || ex) continue;
+    for (int j = W.atom_off + lane; j < W.atom_off + W.n_atoms; j += 32) {
+        if (j == i) continue;
+        int lo = e0, hi = e1;  // j in the sorted exclusion list?
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (a.excl[mid] < j) lo = mid + 1;
+            else hi = mid;
+        }
+        if (lo < e1 && a.excl[lo] == j) continue;
         const float4 xj = a.pos[j];
         const double rx = mimg(xi.x - xj.x, L, h), ry = mimg(xi.y - xj.y, L, h), rz = mimg(xi.z - xj.z, L, h);
-        const double d2 = rx * rx + ry * ry + rz * rz;
-        const double r6 = 1.0 / (d2 * d2 * d2);
-        const double cr = c0 * rx + c1 * ry + c2 * rz;
+        const double r2 = 1.0 / (rx * rx + ry * ry + rz * rz);
+        const double r8 = (r2 * r2) * (r2 * r2);
+        const double cr = (c0 * rx + c1 * ry + c2 * rz) * r8;
         const int kk = a.nbp[ti * a.n_lj_types + a.atype[j].x];
-        atomicAdd(dA + kk, cr * 12.0 * r6 * r6 / d2);
-        atomicAdd(dB + kk, cr * -6.0 * r6 / d2);
+        atomicAdd(dA + kk, 12.0 * cr * (r2 * r2 * r2));
+        atomicAdd(dB + kk, -6.0 * cr);
     }
 }
 
@@ -209,13 +337,17 @@ __global__ void adjoint_14_kernel(AdjointArgs a) {
 }  // namespace
 
 void launch_adjoint(const AdjointArgs &a, cudaStream_t s) {
-    if (a.n_points > 0) {
-        const unsigned blocks = (unsigned)((a.n_points + 127) / 128);
-        adjoint_points_kernel<<<blocks, 128, 0, s>>>(a);
-        adjoint_density_kernel<<<blocks, 128, 0, s>>>(a);
+    if (a.tiles_max > 0) {
+        const unsigned blocks = (unsigned)((long long)a.tiles_max * a.n_windows);
+        adjoint_points_kernel<<<blocks, kAdjThreads, 0, s>>>(a);
+        const size_t smem = (size_t)a.stage * sizeof(float4) + (size_t)(a.stage / 32) * kAdjThreads * sizeof(unsigned);
+        adjoint_density_kernel<<<blocks, kAdjThreads, smem, s>>>(a);
     }
-    if (a.n_adj > 0) adjoint_pairs_kernel<<<(a.n_adj + 63) / 64, 64, 0, s>>>(a);
+    if (a.n_adj > 0) adjoint_pairs_kernel<<<(a.n_adj + 3) / 4, kAdjThreads, 0, s>>>(a);
     if (a.n_dihs > 0) adjoint_14_kernel<<<(a.n_dihs + 127) / 128, 128, 0, s>>>(a);
 }
+
+int adjoint_point_tile() { return kAdjThreads; }
+int adjoint_stage(int max_atoms) { return std::min(kAdjStage, (max_atoms + 31) / 32 * 32); }
 
 }  // namespace isspa

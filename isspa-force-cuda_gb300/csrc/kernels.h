@@ -205,14 +205,16 @@ struct AdjointArgs {
     const int2 *atype;
     const WinDev *win;
     const int *atom_win;
-    long long n_points;
-    const int *point_win;      // [Ptot]
+    int n_windows, tiles_max;  // point tiles of the largest window (adjoint_point_tile() points each)
+    int stage;                 // atoms the density kernel stages at a time (adjoint_stage)
     const float4 *raw_e;       // field pass: E, w
     const float4 *raw_e0;      // field pass: E0, n
     const float4 *q0;          // point positions
     const int *adj_off;        // [n_windows+1] ranges of adj_atoms per window
     const int *adj_atoms;      // atoms with a nonzero weight
     int n_adj;
+    const double *adj_s;       // [n_adj] s_i of the weights c_i = s_i n
+    const double *axis;        // [n_windows][3] unit COM axis n
     const double *cvec;        // [Ntot][3] weights c_i
     const float *rmax, *vtot;
     float f_r0, f_dr, f_inv;
@@ -296,6 +298,8 @@ inline void launch_chain(void (*k)(P...), unsigned grid, unsigned block, cudaStr
 #endif
 
 void launch_adjoint(const AdjointArgs &a, cudaStream_t s);
+int adjoint_point_tile();
+int adjoint_stage(int max_atoms);
 void launch_field(const FieldArgs &a, int split, bool raw, cudaStream_t s);
 void launch_force(const ForceArgs &a, cudaStream_t s);
 // Field and force passes as one launch over the field tiles (split 4, 8 or

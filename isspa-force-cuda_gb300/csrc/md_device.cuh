@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <type_traits>
 
+#include "dfloat.cuh"
 #include "kernels.h"
 #include "philox.h"
 
@@ -199,50 +200,10 @@ __device__ __forceinline__ F3 crossf(F3 a, F3 b) {
 }
 __device__ __forceinline__ F3 scalef(float s, F3 a) { return F3{s * a.x, s * a.y, s * a.z}; }
 
-// Double-float values (hi + lo, two FP32 words) from the error-free
-// transformations of Knuth (TwoSum) and Dekker (TwoProduct, here with an FMA):
-// the bond stretch r0 - |r| and the angle bend theta - theta0 of a geometry
-// near its minimum are small differences of O(1) quantities, which FP32 alone
-// resolves only to ~1e-7 absolute (a relative error of the force that grows
-// as the force vanishes).  Carried in double-float they keep ~1e-7 of their
-// own size; every operation is an FP32 instruction (__fadd_rn / __fmul_rn /
-// fmaf, never contracted or reassociated).
-struct DF {
-    float hi, lo;
-};
-__device__ __forceinline__ DF two_sum(float a, float b) {
-    const float s = __fadd_rn(a, b);
-    const float bb = __fsub_rn(s, a);
-    return DF{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
-}
-__device__ __forceinline__ DF fast_two_sum(float a, float b) {  // |a| >= |b|
-    const float s = __fadd_rn(a, b);
-    return DF{s, __fsub_rn(b, __fsub_rn(s, a))};
-}
-__device__ __forceinline__ DF two_prod(float a, float b) {
-    const float p = __fmul_rn(a, b);
-    return DF{p, fmaf(a, b, -p)};
-}
-__device__ __forceinline__ DF df_add(DF a, DF b) {
-    const DF s = two_sum(a.hi, b.hi);
-    return fast_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo)));
-}
-__device__ __forceinline__ DF df_neg(DF a) { return DF{-a.hi, -a.lo}; }
-__device__ __forceinline__ DF df_mul(DF a, DF b) {
-    const DF p = two_prod(a.hi, b.hi);
-    return fast_two_sum(p.hi, fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, p.lo)));
-}
-// a.b of float vectors, and |a|, in double-float
+// a.b of float vectors in double-float (dfloat.cuh)
 __device__ __forceinline__ DF df_dot(F3 a, F3 b) {
     return df_add(df_add(two_prod(a.x, b.x), two_prod(a.y, b.y)), two_prod(a.z, b.z));
 }
-__device__ __forceinline__ DF df_sqrt(DF a) {  // a > 0; one Newton step on the FP32 root
-    const float s = __fsqrt_rn(a.hi);
-    const float res = __fadd_rn(fmaf(-s, s, a.hi), a.lo);
-    return fast_two_sum(s, __fdiv_rn(res, __fmul_rn(2.0f, s)));
-}
-__device__ __forceinline__ float df_float(DF a) { return __fadd_rn(a.hi, a.lo); }
-
 
 // Fixed-point scatter of one atom's share of a term.
 struct FixAdd {
