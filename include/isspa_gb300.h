@@ -248,11 +248,11 @@ int isspa_engine_info(const isspa_engine *e, int *n_windows, int *n_atoms_total,
 #define ISSPA_SHAPE_COUNT 18
 int isspa_engine_shapes(const isspa_engine *e, int shape[ISSPA_SHAPE_COUNT]);
 /* Autotuner: times every field-pass atom split (per-pair and warp-voted
- * loops, atoms staged by loads or by bulk copies) and, for 1 and 2 receiving
- * atoms per force thread, a set of force-pass chunk lengths (those filling
- * 1..12 whole waves of resident blocks, and powers of two; and long chunks
- * followed by about two waves of short ones; then the voted force loop on the
- * chosen list) on this engine's own
+ * loops, atoms staged by loads or by bulk copies) and, with one receiving atom
+ * per force thread, a set of force-pass chunk lengths (those filling 1..12
+ * whole waves of resident blocks, and powers of two; and long chunks followed
+ * by about two waves of short ones; then the voted force loop on the chosen
+ * list) on this engine's own
  * workload with CUDA events (reps launches each), keeps the fastest of each
  * and reports the result as isspa_engine_shapes does.  When the options leave
  * the integrator, step_pdl, isspa_fused or force_overlap open (0), it then

@@ -1689,15 +1689,18 @@ int isspa_autotune(isspa_engine *e, int reps, int shape[ISSPA_SHAPE_COUNT]) {
         e->field_vote = bestV;
         e->field_tma = bestTma;
         launch_field(e->field_args(), bestS, false, e->stream);
-        // force pass: for 1 and 2 atoms per thread, the chunk lengths that fill
-        // 1..12 whole waves of that kernel's resident blocks, and powers of two
+        // force pass: the chunk lengths that fill 1..12 whole waves of resident
+        // blocks, and powers of two.  One receiving atom per thread: two can time
+        // a little faster alone (1100 atoms: 129 against 134 us) but leave
+        // nothing for force items that start on stamped field tiles, and the
+        // step is slower (211 against 205 us)
         long long maxP = 0;
         for (const WinDev &d : e->win_h) maxP = std::max(maxP, (long long)d.n_atoms * e->n_mc);
         best = 1e30f;
-        int bestC = e->force_chunk, bestT = e->force_tail, bestA = e->force_apt;
-        for (int apt : {1, 2}) {
-            e->force_apt = apt;
-            const long long slots = (long long)e->n_sms * std::max(1, force_blocks_per_sm(apt));
+        int bestC = e->force_chunk, bestT = e->force_tail;
+        e->force_apt = 1;
+        {
+            const long long slots = (long long)e->n_sms * std::max(1, force_blocks_per_sm(1));
             std::vector<int> cands = {e->default_force_chunk()};
             for (int k = 1; k <= 12; ++k) {
                 long long lo = 32, hi = std::max<long long>(32, std::min<long long>(8192, maxP));
@@ -1730,20 +1733,16 @@ int isspa_autotune(isspa_engine *e, int reps, int shape[ISSPA_SHAPE_COUNT]) {
                     best = ms;
                     bestC = ct.first;
                     bestT = ct.second;
-                    bestA = apt;
                 }
             }
         }
-        e->force_apt = bestA;
         e->set_force_chunk(bestC, bestT);
-        // the voted force loop (one atom per thread) on the chosen work list
+        // the voted force loop on the chosen work list
         e->force_vote = 0;
-        if (bestA == 1) {
-            const float plain = time_it([&] { launch_force(e->force_args(), e->stream); });
-            e->force_vote = 1;
-            const float voted = time_it([&] { launch_force(e->force_args(), e->stream); });
-            e->force_vote = voted < plain ? 1 : 0;
-        }
+        const float plain = time_it([&] { launch_force(e->force_args(), e->stream); });
+        e->force_vote = 1;
+        const float voted = time_it([&] { launch_force(e->force_args(), e->stream); });
+        e->force_vote = voted < plain ? 1 : 0;
         // nonbond pass: partner stretches per item (results do not move)
         if (e->opt.nonbond_terms && e->n_nb_items > 0 && !e->cutoff) {
             int maxN = 0;

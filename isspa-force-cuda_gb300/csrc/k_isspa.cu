@@ -38,20 +38,28 @@ constexpr int kForceThreads = 128;
 // <P1>, <P2>, <P3> of a Langevin dipole in a field of magnitude x.  Below 5
 // the ratios i_l/i_(l-1) of modified spherical Bessel functions are taken from
 // their backward continued fraction r_l = x / (2l+1 + x r_(l+1)) (all terms
-// positive, no cancellation); above, the closed forms of the reference
-// (isspa_force_cuda.cu:270-273, 283, 287) are exact to float rounding.
+// positive, no cancellation), carried as numerators and denominators, A_l =
+// x B_(l+1), B_l = (2l+1) B_(l+1) + x A_(l+1), so that <P_m> = r_1 ... r_m =
+// x^m B_(m+1) / B_1 takes one division instead of a chain of twelve (the
+// epilogue is one warp of the block on its own, with the others gone);
+// above, the closed forms of the reference (isspa_force_cuda.cu:270-273, 283,
+// 287) are exact to float rounding.
 __device__ __forceinline__ void langevin3(float x, float &p1, float &p2, float &p3) {
     if (x < 5.0f) {
-        float r = 0.0f, r2 = 0.0f, r3 = 0.0f;
+        float A = 0.0f, B = 1.0f, b2 = 1.0f, b3 = 1.0f, b4 = 1.0f;
 #pragma unroll
         for (int l = 12; l >= 1; --l) {
-            r = __fdiv_rn(x, (float)(2 * l + 1) + x * r);
-            if (l == 3) r3 = r;
-            if (l == 2) r2 = r;
+            const float nb = fmaf(x, A, (float)(2 * l + 1) * B);
+            A = x * B;
+            B = nb;
+            if (l == 4) b4 = B;
+            if (l == 3) b3 = B;
+            if (l == 2) b2 = B;
         }
-        p1 = r;
-        p2 = r * r2;
-        p3 = p2 * r3;
+        const float q = __fdiv_rn(x, B);
+        p1 = q * b2;
+        p2 = q * (x * b3);
+        p3 = q * (x * (x * b4));
     } else {
         const float c = 1.0f / tanhf(x);
         const float ix = 1.0f / x;
@@ -62,25 +70,18 @@ __device__ __forceinline__ void langevin3(float x, float &p1, float &p2, float &
     }
 }
 
-// MC point p (index within its window) of `owner` at position xa with radius
-// rm: uniform in the ball r^2 < 0.99 (isspa_force_cuda.cu:92-100).
-__device__ __forceinline__ void mc_point(uint32_t p, uint32_t window, uint32_t step, uint32_t k0,
-                                         uint32_t k1, float4 xa, float rm, float &px, float &py,
-                                         float &pz) {
-    float mx = 0.5f, my = 0.0f, mz = 0.0f;
-    for (uint32_t att = 0; att < 64u; ++att) {
-        u32x4 o = philox4x32_10(u32x4{p, att, step, (window << 8) | 0u}, k0, k1);
-        float x = __fmaf_rn(2.0f, u01(o.x), -1.0f);
-        float y = __fmaf_rn(2.0f, u01(o.y), -1.0f);
-        float z = __fmaf_rn(2.0f, u01(o.z), -1.0f);
-        if (dist2f(x, y, z) < 0.99f) {
-            mx = x; my = y; mz = z;
-            break;
-        }
-    }
-    px = __fmaf_rn(mx, rm, xa.x);
-    py = __fmaf_rn(my, rm, xa.y);
-    pz = __fmaf_rn(mz, rm, xa.z);
+// Attempt `att` at MC point p (index within its window): a point of the cube
+// [-1, 1)^3, accepted inside the ball r^2 < 0.99 (isspa_force_cuda.cu:92-100).
+// The point is the first accepted attempt of 64; should none be, the fixed
+// offset (0.5, 0, 0).
+constexpr uint32_t kAttempts = 64;
+__device__ __forceinline__ bool mc_attempt(uint32_t p, uint32_t window, uint32_t step, uint32_t k0, uint32_t k1,
+                                           uint32_t att, float &x, float &y, float &z) {
+    const u32x4 o = philox4x32_10(u32x4{p, att, step, (window << 8) | 0u}, k0, k1);
+    x = __fmaf_rn(2.0f, u01(o.x), -1.0f);
+    y = __fmaf_rn(2.0f, u01(o.y), -1.0f);
+    z = __fmaf_rn(2.0f, u01(o.z), -1.0f);
+    return dist2f(x, y, z) < 0.99f;
 }
 
 // 1-D bulk copies (cp.async.bulk, the TMA engine's untiled form) from global
@@ -156,7 +157,8 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, P
     __shared__ alignas(8) unsigned long long s_bar[2];
     __shared__ float s_red[S > 1 ? 8 : 1][kT];
     constexpr bool kShareDraws = GEN && S >= 4;
-    __shared__ float s_pt[3][kShareDraws ? kT / S : 1];  // the block's points, drawn once
+    __shared__ float s_try[kShareDraws ? S : 1][3][kShareDraws ? 32 : 1];  // a batch of attempts at the points
+    __shared__ unsigned s_ok[kShareDraws ? S : 1];
 
     const int4 tile = a.tiles[tile_index];
     const WinDev W = a.win[tile.x];
@@ -166,7 +168,8 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, P
     const bool valid = slot < tile.z;
     const long long pg = tile.y + (valid ? slot : tile.z - 1);  // global point
     const long long pw = pg - W.point_off;                        // point within window
-    const int owner = W.atom_off + (int)(pw / a.n_mc);
+    // (a window's points number less than 2^31: a 32-bit division)
+    const int owner = W.atom_off + (int)((uint32_t)pw / (uint32_t)a.n_mc);
     const float4 xo = a.pos[owner];
     const float rm = __ldg(a.rmax + a.atype[owner].y);
     const float rm2 = __fmul_rn(rm, rm);
@@ -209,30 +212,60 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, P
     }
 
     float px, py, pz;
-    if (kShareDraws) {
-        // one warp of each group draws the group's 32 points (rejection
-        // sampling, divergent attempt counts); the other S-1 warps wait at the
-        // barrier instead of repeating the draws on issue slots the SM needs
-        // (1100 atoms, S = 8: 0.0876 against 0.0925 ms per launch; with S = 2
-        // the barrier costs more than the one repeated draw saves)
-        if (sp == 0) {
-            mc_point((uint32_t)pw, (uint32_t)tile.x, *a.step_ptr, a.seed_lo, a.seed_hi, xo, rm, px, py, pz);
-            s_pt[0][slot] = px;
-            s_pt[1][slot] = py;
-            s_pt[2][slot] = pz;
-        }
-        __syncthreads();
-        px = s_pt[0][slot];
-        py = s_pt[1][slot];
-        pz = s_pt[2][slot];
-    } else {
-        if (GEN) {
-            mc_point((uint32_t)pw, (uint32_t)tile.x, *a.step_ptr, a.seed_lo, a.seed_hi, xo, rm, px, py, pz);
+    if (GEN) {
+        const uint32_t step = *a.step_ptr;
+        float mx = 0.5f, my = 0.0f, mz = 0.0f;
+        if (kShareDraws) {
+            // S >= 4 has one group of 32 points per block: its S warps make S
+            // attempts at every point at once and the first accepted one
+            // counts (the points of one warp's sequential attempts, bit for
+            // bit), instead of one warp drawing alone for the five or six
+            // attempts of its unluckiest lane while the others wait (1100
+            // atoms, S = 8: barrier stalls 1.9 -> 0.7 warps per issue; 44 atoms,
+            // S = 16, with the Langevin change: 11.4 -> 10.5 us per launch)
+            bool open = true;
+            for (uint32_t att = 0;; att += S) {
+                float x, y, z;
+                const bool ok = mc_attempt((uint32_t)pw, (uint32_t)tile.x, step, a.seed_lo, a.seed_hi, att + sp, x, y, z);
+                s_try[sp][0][lane] = x;
+                s_try[sp][1][lane] = y;
+                s_try[sp][2][lane] = z;
+                const unsigned hits = __ballot_sync(0xffffffffu, ok);
+                if (lane == 0) s_ok[sp] = hits;
+                __syncthreads();  // (the first one also covers the staged round)
+                int s = S;
+#pragma unroll
+                for (int k = S - 1; k >= 0; --k)
+                    if ((s_ok[k] >> lane) & 1u) s = k;
+                if (open && s < S) {
+                    mx = s_try[s][0][lane];
+                    my = s_try[s][1][lane];
+                    mz = s_try[s][2][lane];
+                    open = false;
+                }
+                // every warp sees the same 32 points, so the vote is the block's
+                if (!__any_sync(0xffffffffu, open) || att + S >= kAttempts) break;
+                __syncthreads();  // the batch has been read
+            }
         } else {
-            px = a.pts_in[3 * pg + 0];
-            py = a.pts_in[3 * pg + 1];
-            pz = a.pts_in[3 * pg + 2];
+            for (uint32_t att = 0; att < kAttempts; ++att) {
+                float x, y, z;
+                if (mc_attempt((uint32_t)pw, (uint32_t)tile.x, step, a.seed_lo, a.seed_hi, att, x, y, z)) {
+                    mx = x;
+                    my = y;
+                    mz = z;
+                    break;
+                }
+            }
+            __syncthreads();  // first round staged
         }
+        px = __fmaf_rn(mx, rm, xo.x);
+        py = __fmaf_rn(my, rm, xo.y);
+        pz = __fmaf_rn(mz, rm, xo.z);
+    } else {
+        px = a.pts_in[3 * pg + 0];
+        py = a.pts_in[3 * pg + 1];
+        pz = a.pts_in[3 * pg + 2];
         __syncthreads();  // first round staged
     }
 
@@ -472,6 +505,12 @@ struct ForceShape {
 // (:306-312) folded into the record D) into q per unit -q_i vtot_i, the
 // tabulated mean LJ force (:291-305) into l per unit -vtot_i.  rm2 and frow
 // belong to the atom's type; FAR: the point is known to lie outside rmax.
+// Horner form in g = (E^.r) / r^2 with r^-3 factored out of the whole: four FP32
+// operations fewer than term by term (16 384-atom kind of window, voted loop:
+// 8800 atoms nMC 100 12.63 -> 12.22 ms per launch; 12 windows of 44 to 1100 atoms
+// 542 -> 534 us).  Packing two points into f32x2 instructions was tried again with
+// it and costs more: a packed FMA of three distinct operands takes 4.1 cycles of
+// register reads per SM quarter against 2.3 for two scalar ones.
 template <bool LJ, bool FAR>
 __device__ __forceinline__ void point_force(const float4 *R, float rx, float ry, float rz, float d2, float rm2,
                                             int frow, const ForceArgs &a, float &qx, float &qy, float &qz,
@@ -482,19 +521,16 @@ __device__ __forceinline__ void point_force(const float4 *R, float rx, float ry,
     const float ri = rsqrtf(d2);
     const float ri2 = ri * ri;
     const float ri3 = ri2 * ri;
-    const float ri5 = ri3 * ri2;
     const float4 D = R[inside ? 3 : 4];
     const float w = fmaf(E.x, rx, fmaf(E.y, ry, E.z * rz));
     const float dD = fmaf(D.x, rx, fmaf(D.y, ry, D.z * rz));
     const float g = w * ri2;
-    float X = (w * g) * fmaf(K.y, g, K.x);
-    X = fmaf(3.0f, dD, X) - E.w;
-    X = fmaf(-K.w, g, X);
-    const float cR = X * ri5;
-    const float cE = fmaf(-D.w, ri2, fmaf(K.w, g, K.z) * g) * ri3;
-    qx = fmaf(cR, rx, fmaf(-cE, E.x, fmaf(-ri3, D.x, qx)));
-    qy = fmaf(cR, ry, fmaf(-cE, E.y, fmaf(-ri3, D.y, qy)));
-    qz = fmaf(cR, rz, fmaf(-cE, E.z, fmaf(-ri3, D.z, qz)));
+    const float X = fmaf(g, fmaf(w, fmaf(K.y, g, K.x), -K.w), fmaf(3.0f, dD, -E.w));
+    const float Z = X * ri2;
+    const float Y = fmaf(fmaf(K.w, g, K.z), g, -(D.w * ri2));
+    qx = fmaf(ri3, fmaf(Z, rx, fmaf(-Y, E.x, -D.x)), qx);
+    qy = fmaf(ri3, fmaf(Z, ry, fmaf(-Y, E.y, -D.y)), qy);
+    qz = fmaf(ri3, fmaf(Z, rz, fmaf(-Y, E.z, -D.z)), qz);
     if (LJ && inside) {
         const float dist = __fsqrt_rn(d2);
         const int bin = (int)__fmaf_rn(__fsub_rn(dist, a.f_r0), a.f_inv, 0.5f);
