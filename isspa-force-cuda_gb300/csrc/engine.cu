@@ -111,6 +111,13 @@ struct isspa_engine {
     int4 *nb_items = nullptr;
     int *nb_nj = nullptr;
     int n_nb_items = 0, nb_chunk = 0, n_sms = 0;
+    // nonbond items of the merged step (built on first use for a field split)
+    int4 *mg_items = nullptr;
+    int *mg_nj = nullptr;
+    int n_mg_items = 0, mg_split = 0;
+    unsigned long long *mg_copies = nullptr;  // more accumulators for its field tiles
+    int mg_n_copies = 1;
+    bool mg_off = false;  // their buffers did not fit: the branched step runs
     // cutoff mode of the nonbond pass (nonbond_cutoff > 0): Verlet list over cell lists
     bool cutoff = false;
     float nb_cut2 = 0.f, nb_list2 = 0.f, nb_half_skin2 = 0.f;
@@ -328,10 +335,7 @@ struct isspa_engine {
     // Nonbond work items, partner-chunk-major: blocks that run together add
     // into different receiving tiles.  Per-stage sums start at multiples of
     // 128 partners from the window's first atom, so J moves no result.
-    void set_nonbond_chunk(int J) {
-        J = std::max(128, ((J + 127) / 128) * 128);
-        std::vector<int4> items;
-        std::vector<int> nj;
+    void nonbond_items(int J, std::vector<int4> &items, std::vector<int> &nj) const {
         for (int w : order) {
             const WinDev &d = win_h[w];
             for (int j = 0; j < d.n_atoms; j += J)
@@ -340,6 +344,12 @@ struct isspa_engine {
                     nj.push_back(std::min(J, d.n_atoms - j));
                 }
         }
+    }
+    void set_nonbond_chunk(int J) {
+        J = std::max(128, ((J + 127) / 128) * 128);
+        std::vector<int4> items;
+        std::vector<int> nj;
+        nonbond_items(J, items, nj);
         release(nb_items);
         release(nb_nj);
         nb_items = upload(items);
@@ -638,6 +648,65 @@ struct isspa_engine {
     }
     bool overlap() const { return force_overlap == 1 && overlap_ok(); }
 
+    // The merged step: the fused launch's engines with separate integration,
+    // all pairs, an LJ table that fits, and at most an atom per thread of its
+    // integrating block.  Beyond that the integrator takes turns and the
+    // branched graph catches up: twelve windows of 44 atoms 13.7 against 14.4 us
+    // merged, four of 132 atoms 23.0 against 22.7; one of 506 atoms 42.0 against
+    // 43.0.  (A split of 4 never timed best and keeps the branched graph.)
+    bool merged() const {
+        return !mg_off && fused() && field_split >= 8 && integrator == 1 && !cutoff &&
+               n_lj_types <= kMergedMaxLjTypes && n_atoms <= merged_threads(field_split);
+    }
+    // before a capture (allocates): the merged step's nonbond items
+    void prepare_merged() {
+        if (!merged() || mg_split == field_split) return;
+        std::vector<int4> items;
+        std::vector<int> nj;
+        nonbond_items(merged_nonbond_partners(field_split), items, nj);
+        release(mg_items);
+        release(mg_nj);
+        release(mg_copies);
+        // about 16 tiles of a window per accumulator, as far as that is worth
+        // the integrator's extra reads (ADI2, 138 tiles: the tiles' fence and
+        // count take 0.6-1.0 us with four or eight, 1.7 with one)
+        mg_n_copies = std::max(1, std::min(kMergedCopies, n_field_tiles / n_windows / 16));
+        try {
+            mg_items = upload(items);
+            mg_nj = upload(nj);
+            mg_copies = alloc<unsigned long long>(mg_copy_words());
+            ck(cudaMemset(mg_copies, 0, sizeof(unsigned long long) * mg_copy_words()));
+            ck(cudaStreamSynchronize(0));
+        } catch (const Fail &f) {
+            if (f.code != ISSPA_ERR_NOMEM) throw;
+            mg_off = true;
+            return;
+        }
+        n_mg_items = (int)items.size();
+        mg_split = field_split;
+        ck(launch_merged_step(merged_args(), field_split, stream, true));
+    }
+    size_t mg_copy_words() const { return 3 * (size_t)n_atoms * (mg_n_copies - 1); }
+    MergedArgs merged_args() const {
+        MergedArgs m{};
+        m.field = field_args();
+        m.force = force_args();
+        m.nonbond = nonbond_args();
+        m.nonbond.items = mg_items;
+        m.nonbond.items_nj = mg_nj;
+        m.nonbond.n_items = opt.nonbond_terms ? n_mg_items : 0;
+        m.bonded = bonded_args(1, 1, 1);
+        m.us = umbrella_args();
+        m.lf = leapfrog_args();
+        const long long t = merged_threads(field_split);
+        m.n_bonded_blocks = (int)(((long long)n_bonds + n_angles + n_dihs + t - 1) / t);
+        m.n_copies = mg_n_copies;
+        m.copies = mg_copies;
+        m.n_gtab = n_itypes * (n_g - 1);
+        m.n_ftab = n_itypes * n_f;
+        return m;
+    }
+
     // ---------------------------------------------------------- sequences
     void enqueue_isspa(cudaStream_t s, bool raw = false) {
         if (!raw && fused()) {
@@ -656,6 +725,7 @@ struct isspa_engine {
     }
     // Which kernels a step launches (the wrappers skip empty work lists).
     bool launches(int k) const {
+        if (merged()) return k == ISSPA_K_STEP;
         const bool one = integrator == 3;
         switch (k) {
             case ISSPA_K_FIELD: return !one && opt.isspa_terms && n_field_tiles > 0;
@@ -685,6 +755,12 @@ struct isspa_engine {
         if (integrator == 3) {  // the whole step in one cooperative kernel
             mark(ISSPA_K_STEP, 0, stream);
             if (n_atoms > 0) ck(launch_step(step_args(), step_grid(), stream));
+            mark(ISSPA_K_STEP, 1, stream);
+            return;
+        }
+        if (merged()) {
+            mark(ISSPA_K_STEP, 0, stream);
+            ck(launch_merged_step(merged_args(), field_split, stream, false));
             mark(ISSPA_K_STEP, 1, stream);
             return;
         }
@@ -753,6 +829,7 @@ struct isspa_engine {
     cudaEvent_t kev[2 * ISSPA_K_COUNT] = {};
     cudaGraphExec_t graph_timed = nullptr;
     cudaGraphExec_t capture(int nsteps, bool timed = false) {
+        prepare_merged();
         cudaGraph_t g = nullptr;
         ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         try {
@@ -783,6 +860,7 @@ struct isspa_engine {
                                     bool has_out) {
         for (const HostStepGraph &h : host_graphs)
             if (std::equal(h.key, h.key + 5, key)) return h.exec;
+        prepare_merged();
         cudaGraph_t g = nullptr;
         ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         try {
@@ -819,6 +897,7 @@ struct isspa_engine {
     }
     void run_steps(int nsteps) {
         if (!opt.use_graph) {
+            prepare_merged();
             for (int k = 0; k < nsteps; ++k) enqueue_step_forked();
             ck(cudaGetLastError());
             return;
@@ -1742,7 +1821,9 @@ int isspa_autotune(isspa_engine *e, int reps, int shape[ISSPA_SHAPE_COUNT]) {
         const float plain = time_it([&] { launch_force(e->force_args(), e->stream); });
         e->force_vote = 1;
         const float voted = time_it([&] { launch_force(e->force_args(), e->stream); });
-        e->force_vote = voted < plain ? 1 : 0;
+        // (in the step, among other branches' blocks, it costs about a per cent
+        // where the two time equal alone)
+        e->force_vote = voted < 0.985f * plain ? 1 : 0;
         // nonbond pass: partner stretches per item (results do not move)
         if (e->opt.nonbond_terms && e->n_nb_items > 0 && !e->cutoff) {
             int maxN = 0;
@@ -2021,9 +2102,11 @@ int isspa_device_status(isspa_engine *e, int reset) {
         cudaGetLastError();
         return ISSPA_ERR_CUDA;
     }
-    // a grid barrier that gave up leaves its words mid-count: reset them with the status
+    // a grid barrier or a merged step that gave up leaves its count: reset with the status
     if (reset && (cudaMemsetAsync(e->status, 0, sizeof(int), e->stream) != cudaSuccess ||
-                  ((st & kStatusTimeout) && cudaMemsetAsync(e->bar, 0, 2 * sizeof(unsigned int), e->stream) != cudaSuccess) ||
+                  ((st & kStatusTimeout) && (cudaMemsetAsync(e->bar, 0, 2 * sizeof(unsigned int), e->stream) != cudaSuccess ||
+                                             cudaMemsetAsync(e->d_done, 0, sizeof(unsigned int), e->stream) != cudaSuccess ||
+                                             (e->mg_copies && cudaMemsetAsync(e->mg_copies, 0, sizeof(unsigned long long) * e->mg_copy_words(), e->stream) != cudaSuccess))) ||
                   cudaStreamSynchronize(e->stream) != cudaSuccess)) {
         cudaGetLastError();
         return ISSPA_ERR_CUDA;

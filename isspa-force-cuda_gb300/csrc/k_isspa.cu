@@ -34,6 +34,7 @@ namespace {
 
 constexpr int kFieldThreads = 128;
 constexpr int kForceThreads = 128;
+constexpr int kMergedMaxAB = 1024;  // LJ type pairs of a merged step (up to 32 LJ types)
 
 // <P1>, <P2>, <P3> of a Langevin dipole in a field of magnitude x.  Below 5
 // the ratios i_l/i_(l-1) of modified spherical Bessel functions are taken from
@@ -142,23 +143,47 @@ struct FieldShape {
 // FUSE: the tile's point records are also left in s_rec[slot] for a force
 // phase of the same block (which follows a barrier after this function; no
 // barrier of this function comes after a thread's early return).
-template <int S, bool GEN, bool RAW, bool VOTE, bool TMA = false, bool FUSE = false>
-__device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, PointRec *s_rec = nullptr) {
-    static_assert(!FUSE || (GEN && !RAW && !TMA), "the fused pass draws its points and stages by loads");
-    constexpr int kT = FieldShape<S>::kThreads;
+// `wait` is called once what does not move between steps has been read, before
+// the first position is.
+template <int S, bool GEN, bool TMA>
+struct FieldSmem {
+    static constexpr int kT = FieldShape<S>::kThreads;
     // atoms staged per round: four per thread below a split of 4, so the
     // warps' compute phases between barriers are four times longer (64 windows
     // at split 1: 1.779 against 1.808 ms per launch; at split 8 one per thread
     // measured faster); a multiple of S either way, so each warp still visits
     // its atoms (j = sp mod S) in increasing order, whatever the round length
-    constexpr int kA = TMA ? 128 : (S >= 4 ? kT : 4 * kT);
-    __shared__ alignas(16) float4 s_atom[TMA ? 2 : 1][kA];
-    __shared__ int s_row[TMA ? 1 : kA];
-    __shared__ alignas(8) unsigned long long s_bar[2];
-    __shared__ float s_red[S > 1 ? 8 : 1][kT];
-    constexpr bool kShareDraws = GEN && S >= 4;
-    __shared__ float s_try[kShareDraws ? S : 1][3][kShareDraws ? 32 : 1];  // a batch of attempts at the points
-    __shared__ unsigned s_ok[kShareDraws ? S : 1];
+    static constexpr int kA = TMA ? 128 : (S >= 4 ? kT : 4 * kT);
+    static constexpr bool kShareDraws = GEN && S >= 4;
+    alignas(16) float4 atom[TMA ? 2 : 1][kA];
+    int row[TMA ? 1 : kA];
+    alignas(8) unsigned long long bar[2];
+    alignas(16) float red[S > 1 ? 8 : 1][kT];
+    float attempt[kShareDraws ? S : 1][3][kShareDraws ? 32 : 1];  // a batch of attempts at the points
+    unsigned ok[kShareDraws ? S : 1];
+};
+// A table entry: through the read-only path, or from a copy in shared memory.
+template <bool SMEM, class T>
+__device__ __forceinline__ T table_entry(const T *p) {
+    if (SMEM) return *p;
+    return __ldg(p);
+}
+struct NoWait {
+    __device__ void operator()() const {}
+};
+template <int S, bool GEN, bool RAW, bool VOTE, bool TMA = false, bool FUSE = false, bool TS = false, class Wait = NoWait>
+__device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, FieldSmem<S, GEN, TMA> &sm,
+                                           PointRec *s_rec = nullptr, const Wait &wait = Wait{}) {
+    static_assert(!FUSE || (GEN && !RAW && !TMA), "the fused pass draws its points and stages by loads");
+    using Smem = FieldSmem<S, GEN, TMA>;
+    constexpr int kT = Smem::kT, kA = Smem::kA;
+    constexpr bool kShareDraws = Smem::kShareDraws;
+    auto &s_atom = sm.atom;
+    auto &s_row = sm.row;
+    auto &s_bar = sm.bar;
+    auto &s_red = sm.red;
+    auto &s_try = sm.attempt;
+    auto &s_ok = sm.ok;
 
     const int4 tile = a.tiles[tile_index];
     const WinDev W = a.win[tile.x];
@@ -170,12 +195,20 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, P
     const long long pw = pg - W.point_off;                        // point within window
     // (a window's points number less than 2^31: a 32-bit division)
     const int owner = W.atom_off + (int)((uint32_t)pw / (uint32_t)a.n_mc);
-    const float4 xo = a.pos[owner];
     const float rm = __ldg(a.rmax + a.atype[owner].y);
     const float rm2 = __fmul_rn(rm, rm);
     const float L = W.box, h = W.hbox;
-
     const int nb = a.n_gbins;
+    auto stage_types = [&](int j0, int jn) {  // table rows of atoms [j0, j0 + jn)
+        if (!TMA)
+            for (int i = threadIdx.x; i < jn; i += kT) s_row[i] = a.atype[W.atom_off + j0 + i].y * nb;
+    };
+    stage_types(0, min(kA, W.n_atoms));
+    wait();
+    uint32_t step = 0;
+    if (GEN) step = *a.step_ptr;
+    const float4 xo = a.pos[owner];
+
     const int n_rounds = (W.n_atoms + kA - 1) / kA;
     // one round of the window's atoms into shared memory: [j0, j0 + jn)
     auto stage_round = [&](int j0, int jn) {
@@ -184,7 +217,6 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, P
             float4 xj = a.pos[j];
             xj.w = a.e0 * xj.w;  // e0*q (isspa_force_cuda.cu:179, :183)
             s_atom[0][i] = xj;
-            s_row[i] = a.atype[j].y * nb;
         };
         if (kA == kT) {
             if (threadIdx.x < jn) stage(threadIdx.x);
@@ -213,7 +245,6 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, P
 
     float px, py, pz;
     if (GEN) {
-        const uint32_t step = *a.step_ptr;
         float mx = 0.5f, my = 0.0f, mz = 0.0f;
         if (kShareDraws) {
             // S >= 4 has one group of 32 points per block: its S warps make S
@@ -309,7 +340,7 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, P
                 w = 0.0f;
             } else if (bin < nb) {
                 const int row = TMA ? __ldg(&a.atype[W.atom_off + jbase + k].y) * nb : s_row[k];
-                const float4 t = __ldg(a.gtab + row + bin);
+                const float4 t = table_entry<TS>(a.gtab + row + bin);
                 const float fg = (dist - fmaf((float)bin, g_dr, g_r0)) * g_inv;
                 w *= fmaf(fg, t.y - t.x, t.x);
                 const float fe = (dist - fmaf((float)bin, e_dr, e_r0)) * e_inv;
@@ -346,6 +377,7 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, P
             }
         } else if (j0 > 0) {
             __syncthreads();  // the previous round has been read
+            stage_types(j0, jn);
             stage_round(j0, jn);
             __syncthreads();
         }
@@ -403,18 +435,50 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, P
         s_red[6][threadIdx.x] = fy;
         s_red[7][threadIdx.x] = fz;
         __syncthreads();
-        if (sp != 0) return;
+        if (S >= 4) {
+            // one group of points per block: the warps share the eight sums
+            // (in the order of the partial sums)
+            for (int q = sp; q < 8; q += S) {
+                float v = s_red[q][lane];
+                if (q == 0) {
 #pragma unroll
-        for (int s = 1; s < S; ++s) {
-            const int o = (grp * S + s) * 32 + lane;
-            w *= s_red[0][o];
-            n += __float_as_int(s_red[1][o]);
-            ex += s_red[2][o];
-            ey += s_red[3][o];
-            ez += s_red[4][o];
-            fx += s_red[5][o];
-            fy += s_red[6][o];
-            fz += s_red[7][o];
+                    for (int s = 1; s < S; ++s) v *= s_red[q][s * 32 + lane];
+                } else if (q == 1) {
+                    int c = __float_as_int(v);
+#pragma unroll
+                    for (int s = 1; s < S; ++s) c += __float_as_int(s_red[q][s * 32 + lane]);
+                    v = __int_as_float(c);
+                } else {
+#pragma unroll
+                    for (int s = 1; s < S; ++s) v += s_red[q][s * 32 + lane];
+                }
+                s_red[q][lane] = v;  // (no other warp reads this row)
+            }
+            __syncthreads();
+        }
+        if (sp != 0) return;
+        if (S >= 4) {
+            w = s_red[0][lane];
+            n = __float_as_int(s_red[1][lane]);
+            ex = s_red[2][lane];
+            ey = s_red[3][lane];
+            ez = s_red[4][lane];
+            fx = s_red[5][lane];
+            fy = s_red[6][lane];
+            fz = s_red[7][lane];
+        } else {
+#pragma unroll
+            for (int s = 1; s < S; ++s) {
+                const int o = (grp * S + s) * 32 + lane;
+                w *= s_red[0][o];
+                n += __float_as_int(s_red[1][o]);
+                ex += s_red[2][o];
+                ey += s_red[3][o];
+                ez += s_red[4][o];
+                fx += s_red[5][o];
+                fy += s_red[6][o];
+                fz += s_red[7][o];
+            }
         }
     }
     if (!valid) return;
@@ -463,11 +527,6 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, P
     }
 }
 
-__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int *p) {
-    unsigned int v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 __device__ __forceinline__ void st_release_u32(unsigned int *p, unsigned int v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -480,7 +539,8 @@ __global__ void __launch_bounds__(FieldShape<S>::kThreads) field_kernel(FieldArg
     // block's exit does not wait on it
     __shared__ unsigned int s_stamp;
     if (a.tile_flag && threadIdx.x == 0) s_stamp = *a.ov_epoch + 1u;
-    field_tile<S, GEN, RAW, VOTE, TMA>(a, blockIdx.x);
+    __shared__ FieldSmem<S, GEN, TMA> sm;
+    field_tile<S, GEN, RAW, VOTE, TMA>(a, blockIdx.x, sm);
     if (a.tile_flag) {
         // the tile's records are written: the barrier orders every thread's
         // stores before thread 0's release, which the force items acquire
@@ -511,7 +571,7 @@ struct ForceShape {
 // 542 -> 534 us).  Packing two points into f32x2 instructions was tried again with
 // it and costs more: a packed FMA of three distinct operands takes 4.1 cycles of
 // register reads per SM quarter against 2.3 for two scalar ones.
-template <bool LJ, bool FAR>
+template <bool LJ, bool FAR, bool TS = false>
 __device__ __forceinline__ void point_force(const float4 *R, float rx, float ry, float rz, float d2, float rm2,
                                             int frow, const ForceArgs &a, float &qx, float &qy, float &qz,
                                             float &lx, float &ly, float &lz) {
@@ -535,7 +595,7 @@ __device__ __forceinline__ void point_force(const float4 *R, float rx, float ry,
         const float dist = __fsqrt_rn(d2);
         const int bin = (int)__fmaf_rn(__fsub_rn(dist, a.f_r0), a.f_inv, 0.5f);
         if (bin >= 0 && bin < a.n_f) {
-            const float2 tv = __ldg(a.ftab + frow + bin);
+            const float2 tv = table_entry<TS>(a.ftab + frow + bin);
             const float fr = (dist - fmaf((float)bin, a.f_dr, a.f_r0)) * a.f_inv;
             const float fv = fmaf(fr, tv.y - tv.x, tv.x) * R[0].w * ri;
             lx = fmaf(fv, rx, lx);
@@ -708,51 +768,83 @@ __global__ void __launch_bounds__(ForceShape<A>::kThreads, VOTE ? 8 : ForceShape
 // consecutive points, G = min(np, threads / atoms) (at least 1), so small
 // windows keep the block's threads busy; each pair runs the force pass's
 // per-pair arithmetic and sums its group in FP32.  The groups' fixed-point
-// values meet in shared memory (s_acc, windows of up to kFusedSmemAtoms
-// atoms), so the block adds one set of global atomics per atom: every block
-// of a small window adds into the same few hundred words, and per-group
-// global atomics queued on them.
-constexpr int kFusedSmemAtoms = 512;
-template <bool LJ>
-__device__ __forceinline__ void tile_point_forces(const ForceArgs &a, const WinDev &W, const PointRec *s_rec,
-                                                  int np, unsigned long long *s_acc) {
-    const bool smem = W.n_atoms <= kFusedSmemAtoms;
+// values meet in shared memory (s_fix), so the block adds one set of global
+// atomics per atom: every block of a small window adds into the same few
+// hundred words, and per-group global atomics queued on them.
+struct TileAtom {  // one (atom, point group) pair's atom: read ahead of the records
+    float4 x;
+    float rm2, vt;
+    int frow, i, grp;
+};
+__device__ __forceinline__ int tile_groups(const WinDev &W, int np) {
+    return max(1, min(np, (int)blockDim.x / max(W.n_atoms, 1)));
+}
+__device__ __forceinline__ TileAtom tile_atom(const ForceArgs &a, const WinDev &W, int idx) {
+    TileAtom q;
+    q.grp = (uint32_t)idx / (uint32_t)W.n_atoms;
+    q.i = idx - q.grp * W.n_atoms;
+    const int ity = a.atype[W.atom_off + q.i].y;
+    const float rm = __ldg(a.rmax + ity);
+    q.rm2 = __fmul_rn(rm, rm);
+    q.frow = ity * a.n_f;
+    q.vt = __ldg(a.vtot + ity);
+    return q;
+}
+template <bool LJ, bool TS>
+__device__ __forceinline__ bool tile_pair_force(const ForceArgs &a, const WinDev &W, const PointRec *s_rec, int np,
+                                                int per, const TileAtom &q, long long f[3]) {
     const float L = W.box, h = W.hbox;
-    const int n = W.n_atoms;
-    const int G = max(1, min(np, (int)blockDim.x / max(n, 1)));
-    const int per = (np + G - 1) / G;
-    for (int idx = threadIdx.x; idx < n * G; idx += blockDim.x) {
-        const int i = idx % n, grp = idx / n;
-        const int k0 = grp * per, k1 = min(np, k0 + per);
-        const int ai = W.atom_off + i;
-        const float4 xi = a.pos[ai];
-        const int ity = a.atype[ai].y;
-        const float rm = __ldg(a.rmax + ity);
-        const float rm2 = __fmul_rn(rm, rm);
-        const int frow = ity * a.n_f;
-        const float vt = __ldg(a.vtot + ity);
-        float qx = 0.f, qy = 0.f, qz = 0.f, lx = 0.f, ly = 0.f, lz = 0.f;
+    const int k0 = q.grp * per, k1 = min(np, k0 + per);
+    float qx = 0.f, qy = 0.f, qz = 0.f, lx = 0.f, ly = 0.f, lz = 0.f;
 #pragma unroll 4
-        for (int k = k0; k < k1; ++k) {
-            const float4 P = s_rec[k].q[0];
-            const float rx = mimg(P.x - xi.x, L, h);
-            const float ry = mimg(P.y - xi.y, L, h);
-            const float rz = mimg(P.z - xi.z, L, h);
-            point_force<LJ, false>(s_rec[k].q, rx, ry, rz, dist2f(rx, ry, rz), rm2, frow, a, qx, qy, qz, lx, ly, lz);
-        }
-        if (k1 <= k0) continue;
-        const float Fx = -vt * fmaf(xi.w, qx, lx);
-        const float Fy = -vt * fmaf(xi.w, qy, ly);
-        const float Fz = -vt * fmaf(xi.w, qz, lz);
-        check_force(a.status, Fx, Fy, Fz);
-        unsigned long long *acc = smem ? s_acc + 3 * i : a.facc + 3 * (long long)ai;
-        atomicAdd(acc + 0, (unsigned long long)to_fix(Fx));
-        atomicAdd(acc + 1, (unsigned long long)to_fix(Fy));
-        atomicAdd(acc + 2, (unsigned long long)to_fix(Fz));
+    for (int k = k0; k < k1; ++k) {
+        const float4 P = s_rec[k].q[0];
+        const float rx = mimg(P.x - q.x.x, L, h);
+        const float ry = mimg(P.y - q.x.y, L, h);
+        const float rz = mimg(P.z - q.x.z, L, h);
+        point_force<LJ, false, TS>(s_rec[k].q, rx, ry, rz, dist2f(rx, ry, rz), q.rm2, q.frow, a, qx, qy, qz, lx, ly, lz);
     }
-    if (!smem) return;
+    const float Fx = -q.vt * fmaf(q.x.w, qx, lx);
+    const float Fy = -q.vt * fmaf(q.x.w, qy, ly);
+    const float Fz = -q.vt * fmaf(q.x.w, qz, lz);
+    check_force(a.status, Fx, Fy, Fz);
+    f[0] = to_fix(Fx);
+    f[1] = to_fix(Fy);
+    f[2] = to_fix(Fz);
+    return k1 > k0;
+}
+// The whole tile, from thread threadIdx.x's first pair (x not yet set where
+// ahead is false); s_fix [3][blockDim.x].
+template <bool LJ, bool TS>
+__device__ __forceinline__ void tile_point_forces(const ForceArgs &a, const WinDev &W, const PointRec *s_rec,
+                                                  int np, const TileAtom &first, long long *s_fix) {
+    const int n = W.n_atoms, T = blockDim.x, t = threadIdx.x;
+    const int G = tile_groups(W, np), per = (np + G - 1) / G;
+    unsigned long long *acc = a.facc + 3 * (long long)W.atom_off;
+    long long f[3] = {0, 0, 0};
+    if (G == 1) {  // an atom per thread and turn
+        for (int i = t; i < n; i += T) {
+            TileAtom q = first;
+            if (i != t) {
+                q = tile_atom(a, W, i);
+                q.x = a.pos[W.atom_off + i];
+            }
+            tile_pair_force<LJ, TS>(a, W, s_rec, np, per, q, f);
+            for (int k = 0; k < 3; ++k) atomicAdd(acc + 3 * i + k, (unsigned long long)f[k]);
+        }
+        return;
+    }
+    if (t < n * G) {
+        tile_pair_force<LJ, TS>(a, W, s_rec, np, per, first, f);  // (an empty group gives zeros)
+        for (int k = 0; k < 3; ++k) s_fix[k * T + t] = f[k];
+    }
     __syncthreads();
-    for (int c = threadIdx.x; c < 3 * n; c += blockDim.x) atomicAdd(a.facc + 3 * (long long)W.atom_off + c, s_acc[c]);
+    for (int c = t; c < 3 * n; c += T) {
+        const int k = (uint32_t)c / (uint32_t)n, i = c - k * n;
+        long long v = 0;
+        for (int g = 0; g < G; ++g) v += s_fix[k * T + g * n + i];
+        atomicAdd(acc + 3 * i + k, (unsigned long long)v);
+    }
 }
 
 // Field and force passes fused for small windows: each block computes its
@@ -762,17 +854,171 @@ __device__ __forceinline__ void tile_point_forces(const ForceArgs &a, const WinD
 // is waited for; one launch per step instead of two, and no record round trip
 // through L2.  Forces equal the separate passes' up to FP32 summation order
 // (sums over a tile's points instead of a force work item's).
+template <int S>
+struct FusedSmem {
+    FieldSmem<S, true, false> f;
+    PointRec rec[FieldShape<S>::kThreads / S];
+    // the force phase's fixed-point sums take the partial field sums' place
+    __device__ __forceinline__ long long *fix() { return reinterpret_cast<long long *>(f.red); }
+};
+template <int S, bool VOTE, bool TS>
+__device__ __forceinline__ void field_force_tile(const FieldArgs &f, const ForceArgs &g, int tile_index,
+                                                 FusedSmem<S> &sm) {
+    const int4 tile = f.tiles[tile_index];
+    const WinDev W = f.win[tile.x];
+    // this thread's first (atom, point group) pair; its position is read with
+    // the tile's own, right after the wait
+    const int idx = min((int)threadIdx.x, W.n_atoms * tile_groups(W, tile.z) - 1);
+    TileAtom first = tile_atom(g, W, idx);
+    field_tile<S, true, false, VOTE, false, true, TS>(f, tile_index, sm.f, sm.rec, [&] {
+        pdl_wait();
+        first.x = g.pos[W.atom_off + first.i];
+    });
+    pdl_trigger();
+    __syncthreads();
+    tile_point_forces<true, TS>(g, W, sm.rec, tile.z, first, sm.fix());
+}
 template <int S, bool VOTE>
 __global__ void __launch_bounds__(FieldShape<S>::kThreads) field_force_kernel(FieldArgs f, ForceArgs g) {
-    pdl_wait();
-    pdl_trigger();
-    __shared__ PointRec s_rec[FieldShape<S>::kThreads / S];
-    __shared__ unsigned long long s_acc[3 * kFusedSmemAtoms];
-    for (int c = threadIdx.x; c < 3 * kFusedSmemAtoms; c += blockDim.x) s_acc[c] = 0ull;
-    field_tile<S, true, false, VOTE, false, true>(f, blockIdx.x, s_rec);  // (its first barrier orders s_acc)
+    __shared__ FusedSmem<S> sm;
+    static_assert(sizeof(sm.f.red) >= 3 * FieldShape<S>::kThreads * sizeof(long long), "the sums fit");
+    field_force_tile<S, VOTE, false>(f, g, blockIdx.x, sm);
+}
+
+// A whole MD step in one ordinary launch, for engines of a few hundred atoms
+// whose step the fused field + force launch bounds: the step's independent
+// chains become blocks of one grid (field tiles with their points' forces,
+// nonbond stages, bonded terms, restraints), all adding into the fixed-point
+// accumulator, and one block integrates every atom once the others have counted
+// themselves done (a bounded wait; no other block waits for any).  Against the branched graph of five kernels a step
+// saves the graph's forks and joins, a kernel boundary, and with programmatic
+// launches the reads of everything that does not move between steps, which run
+// before the wait for the previous step.  Every role is the separate kernels'
+// code, so the trajectory is theirs bit for bit (with the fused launch).
+// Per back-to-back step, the branched graph of the fused launch before and this
+// (best field split): 44 atoms nMC 20 10.6 -> 8.0 us, ADI2 (44 atoms, nMC 100,
+// restrained) 11.3 -> 9.9, 132 atoms 15.8 -> 11.5, 264 atoms 23.7 -> 22.5, four
+// windows of 44 atoms 11.8 -> 8.5.  What is left of a 44-atom step, from
+// %globaltimer: 0.9 us positions and draws, 0.9 atom loop, 0.7 sums and
+// Langevin, 1.4 forces, 0.8 to the integrator's sight (fence, count, poll), 1.3
+// its read of the sums and update, 1.3 to the next step's start -- L2 round
+// trips of half a microsecond each, and branches in the pair loops.
+template <int S>
+struct MergedSmem {
+    union {
+        FusedSmem<S> tile;
+        struct {
+            NonbondSmem nb[FieldShape<S>::kThreads / kNbThreads];
+            float2 ab[kMergedMaxAB];
+        };
+        struct {
+            double red[6 * kUsThreads];
+            double f4[4];
+        };
+    };
+};
+// TS: the field tiles' blocks copy the density / field and force tables into
+// shared memory before the wait (a look-up inside the step is then a shared
+// load instead of an L2 round trip: the caches start the step cold).
+template <int S, bool NB_ALL, bool TS>
+__global__ void __launch_bounds__(FieldShape<S>::kThreads) merged_step_kernel(MergedArgs m) {
+    constexpr int kT = FieldShape<S>::kThreads;
+    extern __shared__ unsigned char s_dyn[];
+    MergedSmem<S> &sm = *reinterpret_cast<MergedSmem<S> *>(s_dyn);
+    int b = blockIdx.x;
+    if (b == 0) {
+        // the integrator: everything but the force is ready when the last of
+        // the other blocks has added its share
+        __shared__ int s_ok;
+        pdl_wait();
+        pdl_trigger();
+        const uint32_t step = *m.lf.step_ptr;
+        LeapfrogAtom first = {};
+        if (threadIdx.x < m.lf.n_atoms) first = leapfrog_prepare(m.lf, threadIdx.x, step);
+        if (threadIdx.x == 0) {
+            s_ok = 1;
+            const unsigned long long t0 = global_ns();
+            while (ld_acquire_u32(m.lf.done_ptr) != gridDim.x - 1)
+                if (global_ns() - t0 > kBarrierWaitNs) {
+                    atomicOr(m.lf.status, kStatusTimeout);
+                    s_ok = 0;
+                    break;
+                }
+        }
+        __syncthreads();
+        if (!s_ok) return;  // (the status reset clears the count)
+        for (int i = threadIdx.x; i < m.lf.n_atoms; i += kT) {
+            // the other copies of the accumulator: read all at once, cleared
+            long long extra[3] = {0, 0, 0}, c[kMergedCopies - 1][3];
+#pragma unroll
+            for (int r = 0; r < kMergedCopies - 1; ++r)
+                for (int k = 0; k < 3; ++k)
+                    c[r][k] = r < m.n_copies - 1
+                                  ? (long long)__ldcg(m.copies + 3 * ((long long)r * m.lf.n_atoms + i) + k)
+                                  : 0;
+#pragma unroll
+            for (int r = 0; r < kMergedCopies - 1; ++r)
+                for (int k = 0; k < 3; ++k) {
+                    extra[k] += c[r][k];
+                    if (r < m.n_copies - 1) m.copies[3 * ((long long)r * m.lf.n_atoms + i) + k] = 0ull;
+                }
+            leapfrog_finish(m.lf, i, i == threadIdx.x ? first : leapfrog_prepare(m.lf, i, step), extra);
+        }
+        if (threadIdx.x == 0) {  // every other block has read the step counter
+            *m.lf.step_ptr = step + 1u;
+            if (m.lf.ov_epoch) ++*m.lf.ov_epoch;
+            *m.lf.done_ptr = 0u;
+        }
+        return;
+    }
+    if (--b < m.field.n_tiles) {
+        FieldArgs f = m.field;
+        ForceArgs g = m.force;
+        if (TS) {
+            auto gt = reinterpret_cast<float4 *>(s_dyn + sizeof(MergedSmem<S>));
+            auto ft = reinterpret_cast<float2 *>(gt + m.n_gtab);
+            for (int k = threadIdx.x; k < m.n_gtab; k += kT) gt[k] = m.field.gtab[k];
+            for (int k = threadIdx.x; k < m.n_ftab; k += kT) ft[k] = m.force.ftab[k];
+            f.gtab = gt;  // (read after the tile's first barrier)
+            g.ftab = ft;
+        }
+        // tiles add into n_copies accumulators in turn: 138 blocks adding into
+        // one copy of a 44-atom window queued on its 132 words
+        if (const int r = b % m.n_copies) g.facc = m.copies + 3 * (long long)(r - 1) * m.lf.n_atoms;
+        field_force_tile<S, false, TS>(f, g, b, sm.tile);
+    } else if ((b -= m.field.n_tiles) < m.nonbond.n_items) {
+        // a block's groups of 128 threads take the stages of its item, which
+        // are summed into fixed point stage by stage in any case
+        for (int k = threadIdx.x; k < m.nonbond.n_lj_types * m.nonbond.n_lj_types; k += kT) sm.ab[k] = m.nonbond.ljab[k];
+        const int g = threadIdx.x / kNbThreads;
+        int4 item = m.nonbond.items[b];
+        const int nj = min(kNbThreads, m.nonbond.items_nj[b] - g * kNbThreads);
+        item.w += g * kNbThreads;
+        if (nj > 0) {
+            nonbond_range<true, NB_ALL, true>(m.nonbond, item, nj, threadIdx.x % kNbThreads, sm.nb[g], sm.ab);
+        } else {
+            __syncthreads();
+            pdl_wait();
+            __syncthreads();
+        }
+        pdl_trigger();
+    } else if ((b -= m.nonbond.n_items) < m.n_bonded_blocks) {
+        pdl_wait();
+        pdl_trigger();
+        bonded_term(m.bonded, (long long)b * kT + threadIdx.x, FixAdd{m.bonded.facc, m.bonded.status});
+    } else {
+        b -= m.n_bonded_blocks;
+        umbrella_window(m.us, m.us.us_windows[b], sm.red, sm.f4, [] {
+            pdl_wait();
+            pdl_trigger();
+        });
+    }
+    // the barrier orders every thread's atomics before thread 0's release
     __syncthreads();
-    const int4 tile = f.tiles[blockIdx.x];
-    tile_point_forces<true>(g, f.win[tile.x], s_rec, tile.z, s_acc);
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(m.lf.done_ptr, 1u);
+    }
 }
 
 // The whole MD step in one cooperative launch, for engines whose step is
@@ -788,13 +1034,14 @@ __global__ void __launch_bounds__(FieldShape<S>::kThreads) field_force_kernel(Fi
 template <bool NB_ALL>
 __global__ void __launch_bounds__(kFieldThreads, 4) step_kernel(StepArgs a) {
     extern __shared__ float2 s_ab[];
+    __shared__ FieldSmem<4, true, false> s_field;
     const uint32_t step = *a.integ.lf.step_ptr;
     if (a.nonbond.n_items > 0) stage_ljab(a.nonbond, s_ab);
     // field tiles and nonbond items as one list over the blocks, so a block
     // left without a tile takes a nonbond item instead of queueing behind one
     const int n1 = a.field.n_tiles + a.nonbond.n_items;
     for (int t = blockIdx.x; t < n1; t += gridDim.x) {
-        if (t < a.field.n_tiles) field_tile<4, true, false, false>(a.field, t);
+        if (t < a.field.n_tiles) field_tile<4, true, false, false>(a.field, t, s_field);
         else nonbond_item<true, NB_ALL>(a.nonbond, t - a.field.n_tiles, s_ab);
     }
     bonded_terms(a.integ.bonded);
@@ -898,6 +1145,35 @@ cudaError_t launch_step(const StepArgs &a, int grid, cudaStream_t s) {
     cfg.numAttrs = 1;
     if (a.nonbond.terms == 7) return cudaLaunchKernelEx(&cfg, step_kernel<true>, a);
     return cudaLaunchKernelEx(&cfg, step_kernel<false>, a);
+}
+
+int merged_threads(int split) { return 32 * split; }
+int merged_nonbond_partners(int split) { return 32 * split; }  // a stage of 128 per group of 128 threads
+
+namespace {
+template <int S, bool TS>
+size_t merged_smem(const MergedArgs &m) {
+    return sizeof(MergedSmem<S>) + (TS ? sizeof(float4) * (size_t)m.n_gtab + sizeof(float2) * (size_t)m.n_ftab : 0);
+}
+// Tables in shared memory while two blocks (a step's and the next one's) fit
+// an SM; 16 types on a 120-point grid take 46 KB beside the block's 36.
+template <int S, bool NB_ALL>
+cudaError_t merged_go(const MergedArgs &m, cudaStream_t s, bool prepare) {
+    constexpr size_t kTwoPerSm = 112 << 10;
+    const bool ts = merged_smem<S, true>(m) <= kTwoPerSm;
+    const size_t smem = ts ? merged_smem<S, true>(m) : merged_smem<S, false>(m);
+    void (*k)(MergedArgs) = ts ? merged_step_kernel<S, NB_ALL, true> : merged_step_kernel<S, NB_ALL, false>;
+    if (prepare) return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTwoPerSm);
+    const unsigned grid = 1 + m.field.n_tiles + m.nonbond.n_items + m.n_bonded_blocks + m.us.n_us_windows;
+    launch_chain_smem(k, grid, FieldShape<S>::kThreads, smem, s, m);
+    return cudaSuccess;
+}
+}  // namespace
+cudaError_t launch_merged_step(const MergedArgs &m, int split, cudaStream_t s, bool prepare) {
+    if (m.lf.n_atoms <= 0) return cudaSuccess;
+    const bool all = m.nonbond.terms == 7;
+    if (split == 16) return all ? merged_go<16, true>(m, s, prepare) : merged_go<16, false>(m, s, prepare);
+    return all ? merged_go<8, true>(m, s, prepare) : merged_go<8, false>(m, s, prepare);
 }
 
 bool field_force_fusable(int split) { return split == 4 || split == 8 || split == 16; }

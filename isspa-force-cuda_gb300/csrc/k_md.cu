@@ -42,15 +42,7 @@ __global__ void bonded_kernel(BondedArgs a) {
 __global__ void __launch_bounds__(kUsThreads) umbrella_kernel(UmbrellaArgs a) {
     __shared__ double s_red[6 * kUsThreads];
     __shared__ double s_f[4];
-    const int w = a.us_windows[blockIdx.x];
-    umbrella_com_block(a, w, s_red, s_f);
-    const WinDev W = a.win[w];
-    for (int b = threadIdx.x; b < W.n_bias; b += kUsThreads) {
-        long long f[3];
-        umbrella_entry_fix(a, W, b, s_f, f);
-        unsigned long long *acc = a.facc + 3 * (long long)a.bias[W.bias_off + b].x;
-        for (int k = 0; k < 3; ++k) atomicAdd(acc + k, (unsigned long long)f[k]);
-    }
+    umbrella_window(a, a.us_windows[blockIdx.x], s_red, s_f, [] {});
 }
 
 // Every block reads the step counter first; the last block to finish

@@ -188,6 +188,20 @@ struct StepArgs {
     IntegratorArgs integ;
 };
 
+// A whole MD step of a small engine in one ordinary launch (see merged_step_kernel).
+struct MergedArgs {
+    FieldArgs field;
+    ForceArgs force;
+    NonbondArgs nonbond;       // items of merged_nonbond_partners() partners
+    BondedArgs bonded;
+    UmbrellaArgs us;
+    LeapfrogArgs lf;
+    int n_bonded_blocks;
+    int n_gtab, n_ftab;        // entries of the packed tables
+    int n_copies;              // accumulators the field tiles add into: lf.facc and n_copies - 1 more
+    unsigned long long *copies;  // [n_copies - 1][n_atoms][3], zero between steps
+};
+
 struct ListArgs {
     const float4 *pos;
     const int *excl_start;
@@ -279,14 +293,16 @@ class PdlScope {
 };
 #ifdef __CUDACC__
 template <class... P, class... A>
-inline void launch_chain(void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, const A &...args) {
+inline void launch_chain_smem(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                              const A &...args) {
     if (!chain_pdl()) {
-        k<<<grid, block, 0, s>>>(args...);
+        k<<<grid, block, smem, s>>>(args...);
         return;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -294,6 +310,10 @@ inline void launch_chain(void (*k)(P...), unsigned grid, unsigned block, cudaStr
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, k, args...);  // a failure is the thread's last error
+}
+template <class... P, class... A>
+inline void launch_chain(void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, const A &...args) {
+    launch_chain_smem(k, grid, block, 0, s, args...);
 }
 #endif
 
@@ -307,6 +327,14 @@ void launch_force(const ForceArgs &a, cudaStream_t s);
 // atom of its window right after their fields are known.
 bool field_force_fusable(int split);
 void launch_field_force(const FieldArgs &f, const ForceArgs &g, int split, cudaStream_t s);
+// The whole step in one launch (field split 4, 8 or 16; blocks of 32 threads per
+// split): its nonbond items hold up to merged_nonbond_partners() partners.
+constexpr int kMergedMaxLjTypes = 32;
+int merged_nonbond_partners(int split);
+int merged_threads(int split);
+constexpr int kMergedCopies = 4;
+// prepare: only sets the kernel's shared-memory limit (before a capture)
+cudaError_t launch_merged_step(const MergedArgs &m, int split, cudaStream_t s, bool prepare);
 void launch_nonbond(const NonbondArgs &a, cudaStream_t s);
 // Cutoff mode: displacement check and (when it trips) the list rebuild; then the pairs.
 void launch_nblist_build(const NbListArgs &a, cudaStream_t s);

@@ -27,18 +27,26 @@ constexpr int kNbMaxAB = 4096;  // LJ type pairs held in shared memory (up to 64
 // of the warp excludes runs without per-pair checks.  SMEM_AB: the LJ (A, B)
 // table of every ordered type pair sits in shared memory (dynamic, nt^2
 // float2) instead of a global gather per pair.  ALL: every term on (mask 7).
-template <bool SMEM_AB, bool ALL>
-__device__ __forceinline__ void nonbond_item(const NonbondArgs &a, int item_index, const float2 *s_ab) {
-    __shared__ float4 s_x[kNbThreads];
-    __shared__ float4 s_c[kNbThreads];  // rmax_j, (2 rmax_j)^2, 8 rmax_j, (1-1/ep)/(24 rmax_j^4)
-    __shared__ int s_t[kNbThreads];
-    const int4 item = a.items[item_index];
-    const int nj = a.items_nj[item_index];
+//
+// The item's thread t of kNbThreads; every thread of the block calls this, with
+// two barriers per stage.  WAIT: a programmatic dependent that waits for the
+// kernel before it here, once everything that does not move between steps
+// (types, exclusions, parameters) has been read.
+struct NonbondSmem {
+    float4 x[kNbThreads];
+    float4 c[kNbThreads];  // rmax_j, (2 rmax_j)^2, 8 rmax_j, (1-1/ep)/(24 rmax_j^4)
+    int t[kNbThreads];
+};
+template <bool SMEM_AB, bool ALL, bool WAIT = false>
+__device__ __forceinline__ void nonbond_range(const NonbondArgs &a, int4 item, int nj, int t, NonbondSmem &sm,
+                                              const float2 *s_ab) {
+    float4 *const s_x = sm.x, *const s_c = sm.c;
+    int *const s_t = sm.t;
     const WinDev W = a.win[item.x];
-    const int t = threadIdx.x;
     const bool active = t < item.z;
     const int i = item.y + (active ? t : 0);
-    const float4 xi = a.pos[i];
+    float4 xi;
+    if (!WAIT) xi = a.pos[i];
     const int nt = a.n_lj_types;
     const int trow = a.atype[i].x * nt;
     const float L = W.box, h = W.hbox;
@@ -76,15 +84,18 @@ __device__ __forceinline__ void nonbond_item(const NonbondArgs &a, int item_inde
         float ax = 0.f, ay = 0.f, az = 0.f;
         __syncthreads();
         if (t < jn) {
-            const int j = jb + t;
-            s_x[t] = a.pos[j];
-            const int2 ty = a.atype[j];
+            const int2 ty = a.atype[jb + t];
             const float rm = __ldg(a.rmax + ty.y);
             const float two = 2.0f * rm;
             const float r2 = rm * rm;
             s_c[t] = make_float4(rm, __fmul_rn(two, two), 8.0f * rm, epf / (24.0f * r2 * r2));
             s_t[t] = ty.x;
         }
+        if (WAIT && j0 == 0) {
+            pdl_wait();
+            xi = a.pos[i];
+        }
+        if (t < jn) s_x[t] = a.pos[jb + t];
         __syncthreads();
         // the pair (i, staged partner k); EX: excluded (IS-SPA correction
         // only).  MASKED: the exclusion bit and the self pair are applied by
@@ -159,6 +170,12 @@ __device__ __forceinline__ void nonbond_item(const NonbondArgs &a, int item_inde
     atomicAdd(acc + 0, (unsigned long long)fxa);
     atomicAdd(acc + 1, (unsigned long long)fya);
     atomicAdd(acc + 2, (unsigned long long)fza);
+}
+
+template <bool SMEM_AB, bool ALL>
+__device__ __forceinline__ void nonbond_item(const NonbondArgs &a, int item_index, const float2 *s_ab) {
+    __shared__ NonbondSmem sm;
+    nonbond_range<SMEM_AB, ALL>(a, a.items[item_index], a.items_nj[item_index], threadIdx.x, sm, s_ab);
 }
 
 // Stages the LJ (A, B) table of every ordered type pair into shared memory
@@ -323,28 +340,53 @@ constexpr int kUsThreads = 256;
 // block in a fixed order (us_force_cuda.cu:14-48, whose __syncthreads only
 // orders a single block); writes the COMs and the CV of the window and returns
 // (in `sf`, on every thread) the minimum-image COM axis r and (|r| - x0)/|r|.
+// `wait` is called once the restraint's lists have been read, before a position is.
+template <class Wait>
 __device__ void umbrella_com_block(const UmbrellaArgs &a, int w, double *s_red /* [6][kUsThreads] */,
-                                   double *sf /* [4], shared */) {
+                                   double *sf /* [4], shared */, const Wait &wait) {
     const WinDev W = a.win[w];
-    double c[6] = {0, 0, 0, 0, 0, 0};
-    for (int b = threadIdx.x; b < W.n_bias; b += blockDim.x) {
-        const int2 e = a.bias[W.bias_off + b];
-        const float4 x = a.pos[e.x];
-        const double m = a.mfrac[W.bias_off + b];
-        const int o = 3 * e.y;
-        c[o + 0] += m * x.x;
-        c[o + 1] += m * x.y;
-        c[o + 2] += m * x.z;
+    int2 e0 = make_int2(0, 0);
+    double m0 = 0.0;
+    if ((int)threadIdx.x < W.n_bias) {
+        e0 = a.bias[W.bias_off + threadIdx.x];
+        m0 = a.mfrac[W.bias_off + threadIdx.x];
     }
-    for (int k = 0; k < 6; ++k) s_red[k * kUsThreads + threadIdx.x] = c[k];
-    for (int t = threadIdx.x + blockDim.x; t < kUsThreads; t += blockDim.x)
-        for (int k = 0; k < 6; ++k) s_red[k * kUsThreads + t] = 0.0;
+    wait();
+    // kUsThreads partial sums whatever the block size
+    for (int t = threadIdx.x; t < kUsThreads; t += blockDim.x) {
+        double c[6] = {0, 0, 0, 0, 0, 0};
+        for (int b = t; b < W.n_bias; b += kUsThreads) {
+            const bool first = b == (int)threadIdx.x;
+            const int2 e = first ? e0 : a.bias[W.bias_off + b];
+            const float4 x = a.pos[e.x];
+            const double m = first ? m0 : a.mfrac[W.bias_off + b];
+            const int o = 3 * e.y;
+            c[o + 0] += m * x.x;
+            c[o + 1] += m * x.y;
+            c[o + 2] += m * x.z;
+        }
+        for (int k = 0; k < 6; ++k) s_red[k * kUsThreads + t] = c[k];
+    }
     __syncthreads();
-    for (int stride = kUsThreads / 2; stride > 0; stride >>= 1) {
-        for (int t = threadIdx.x; t < stride; t += blockDim.x)
-            for (int k = 0; k < 6; ++k) s_red[k * kUsThreads + t] += s_red[k * kUsThreads + t + stride];
-        __syncthreads();
+    // each component's tree (strides 128, 64, ... 1) by one warp in registers: a
+    // shared-memory tree over all six took 3 us of a 44-atom window's 6.3;
+    // partial sums beyond the list are zero
+    for (int k = threadIdx.x >> 5; k < 6; k += blockDim.x >> 5) {
+        const int lane = threadIdx.x & 31;
+        double v[kUsThreads / 32];
+#pragma unroll
+        for (int j = 0; j < kUsThreads / 32; ++j) v[j] = s_red[k * kUsThreads + 32 * j + lane];
+#pragma unroll
+        for (int half = kUsThreads / 64; half > 0; half >>= 1)
+            if (W.n_bias > 32 * half) {
+#pragma unroll
+                for (int j = 0; j < half; ++j) v[j] += v[j + half];
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[0] += __shfl_down_sync(0xffffffffu, v[0], o);
+        if (lane == 0) s_red[k * kUsThreads] = v[0];
     }
+    __syncthreads();
     if (threadIdx.x == 0) {
         const double L = W.box, hh = 0.5 * W.box;
         double r[3];
@@ -379,12 +421,64 @@ __device__ __forceinline__ void umbrella_entry_fix(const UmbrellaArgs &a, const 
 }
 
 
-// Leapfrog of atom i (leapfrog_cuda.cu:33-68) from the accumulated force
-// plus `extra` (fixed point), which it reads through L2 and clears.
+// The restraint of one window by one block: the COMs, then the force on every
+// entry.
+template <class Wait>
+__device__ __forceinline__ void umbrella_window(const UmbrellaArgs &a, int w, double *s_red, double *s_f,
+                                                const Wait &wait) {
+    umbrella_com_block(a, w, s_red, s_f, wait);
+    const WinDev W = a.win[w];
+    for (int b = threadIdx.x; b < W.n_bias; b += blockDim.x) {
+        long long f[3];
+        umbrella_entry_fix(a, W, b, s_f, f);
+        unsigned long long *acc = a.facc + 3 * (long long)a.bias[W.bias_off + b].x;
+        for (int k = 0; k < 3; ++k) atomicAdd(acc + k, (unsigned long long)f[k]);
+    }
+}
 
-__device__ __forceinline__ void leapfrog_atom(const LeapfrogArgs &a, int i, uint32_t step, const long long *extra) {
+// Leapfrog of atom i (leapfrog_cuda.cu:33-68) in two parts: everything but the
+// force (state, parameters, the Andersen draws), then the update from the
+// accumulated force plus `extra` (fixed point), which it reads through L2 and
+// clears.
+struct LeapfrogAtom {
+    float4 x, v;
+    float L, dt, k;        // box, time step, force factor: dt / m, or dt / 2m after a collision
+    float gx, gy, gz, sd;  // collision: normal deviates and the velocity's standard deviation
+    bool hit;
+};
+__device__ __forceinline__ LeapfrogAtom leapfrog_prepare(const LeapfrogArgs &a, int i, uint32_t step) {
+    LeapfrogAtom q;
+    q.v = a.vel[i];
+    q.x = a.pos[i];
     const int w = a.atom_win[i];
     const WinDev W = a.win[w];
+    q.L = W.box;
+    q.dt = W.dt;
+    const uint32_t il = (uint32_t)(i - W.atom_off);
+    const uint32_t ctr3 = ((uint32_t)w << 8) | 1u;
+    const u32x4 o = philox4x32_10(u32x4{il, 0u, step, ctr3}, a.seed_lo, a.seed_hi);
+    const float m = q.v.w;
+    q.hit = u01(o.x) < W.pnu;
+    if (q.hit) {  // Andersen collision (:50-56)
+        const u32x4 g = philox4x32_10(u32x4{il, 1u, step, ctr3}, a.seed_lo, a.seed_hi);
+        const float ra = sqrtf(-2.0f * logf(u01_open0(g.x)));
+        const float rb = sqrtf(-2.0f * logf(u01_open0(g.z)));
+        float s1, c1, s3, c3;
+        sincospif(2.0f * u01_open0(g.y), &s1, &c1);
+        sincospif(2.0f * u01_open0(g.w), &s3, &c3);
+        q.sd = sqrtf(W.kT / m);
+        q.gx = __fmul_rn(ra, c1);
+        q.gy = __fmul_rn(ra, s1);
+        q.gz = __fmul_rn(rb, c3);
+        q.k = W.dt / (2.0f * m);
+    } else {
+        q.gx = q.gy = q.gz = q.sd = 0.0f;
+        q.k = W.dt / m;
+    }
+    return q;
+}
+__device__ __forceinline__ void leapfrog_finish(const LeapfrogArgs &a, int i, const LeapfrogAtom &q,
+                                                const long long *extra) {
     unsigned long long *acc = a.facc + 3 * (long long)i;
     long long s[3] = {(long long)__ldcg(acc + 0), (long long)__ldcg(acc + 1), (long long)__ldcg(acc + 2)};
     if (extra)
@@ -396,35 +490,21 @@ __device__ __forceinline__ void leapfrog_atom(const LeapfrogArgs &a, int i, uint
     acc[1] = 0ull;
     acc[2] = 0ull;
     a.force_out[i] = make_float4(fx, fy, fz, 0.0f);
-    float4 v = a.vel[i];
-    float4 x = a.pos[i];
-    const uint32_t il = (uint32_t)(i - W.atom_off);
-    const uint32_t ctr3 = ((uint32_t)w << 8) | 1u;
-    const u32x4 o = philox4x32_10(u32x4{il, 0u, step, ctr3}, a.seed_lo, a.seed_hi);
-    const float m = v.w;
-    if (u01(o.x) < W.pnu) {  // Andersen collision (:50-56)
-        const u32x4 g = philox4x32_10(u32x4{il, 1u, step, ctr3}, a.seed_lo, a.seed_hi);
-        const float ra = sqrtf(-2.0f * logf(u01_open0(g.x)));
-        const float rb = sqrtf(-2.0f * logf(u01_open0(g.z)));
-        float s1, c1, s3, c3;
-        sincospif(2.0f * u01_open0(g.y), &s1, &c1);
-        sincospif(2.0f * u01_open0(g.w), &s3, &c3);
-        const float sd = sqrtf(W.kT / m);
-        const float hk = W.dt / (2.0f * m);
-        v.x = ra * c1 * sd + fx * hk;
-        v.y = ra * s1 * sd + fy * hk;
-        v.z = rb * c3 * sd + fz * hk;
+    float4 v = q.v, x = q.x;
+    if (q.hit) {
+        v.x = fmaf(q.gx, q.sd, __fmul_rn(fx, q.k));
+        v.y = fmaf(q.gy, q.sd, __fmul_rn(fy, q.k));
+        v.z = fmaf(q.gz, q.sd, __fmul_rn(fz, q.k));
     } else {
-        const float k = W.dt / m;
-        v.x += fx * k;
-        v.y += fy * k;
-        v.z += fz * k;
+        v.x = fmaf(fx, q.k, v.x);
+        v.y = fmaf(fy, q.k, v.y);
+        v.z = fmaf(fz, q.k, v.z);
     }
-    x.x += v.x * W.dt;
-    x.y += v.y * W.dt;
-    x.z += v.z * W.dt;
+    x.x = fmaf(v.x, q.dt, x.x);
+    x.y = fmaf(v.y, q.dt, x.y);
+    x.z = fmaf(v.z, q.dt, x.z);
     // wrap (cuda_vector_routines.h wrap)
-    const float L = W.box;
+    const float L = q.L;
     x.x = x.x > L ? x.x - L : (x.x < 0.0f ? x.x + L : x.x);
     x.y = x.y > L ? x.y - L : (x.y < 0.0f ? x.y + L : x.y);
     x.z = x.z > L ? x.z - L : (x.z < 0.0f ? x.z + L : x.z);
@@ -432,6 +512,15 @@ __device__ __forceinline__ void leapfrog_atom(const LeapfrogArgs &a, int i, uint
         atomicOr(a.status, kStatusNonFinite);
     a.vel[i] = v;
     a.pos[i] = x;
+}
+__device__ __forceinline__ void leapfrog_atom(const LeapfrogArgs &a, int i, uint32_t step, const long long *extra) {
+    leapfrog_finish(a, i, leapfrog_prepare(a, i, step), extra);
+}
+
+__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int *p) {
+    unsigned int v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
 }
 
 // Grid-wide barrier of a cooperative launch (every block resident): arrival
@@ -482,7 +571,7 @@ __device__ __forceinline__ void restraint_coms(const IntegratorArgs &a) {
     __shared__ double s_f[4];
     for (int u = blockIdx.x; u < a.us.n_us_windows; u += gridDim.x) {
         const int w = a.us.us_windows[u];
-        umbrella_com_block(a.us, w, s_red, s_f);
+        umbrella_com_block(a.us, w, s_red, s_f, [] {});
         if (threadIdx.x == 0) {
             a.usf[2 * w] = make_double2(s_f[0], s_f[1]);
             a.usf[2 * w + 1] = make_double2(s_f[2], s_f[3]);
