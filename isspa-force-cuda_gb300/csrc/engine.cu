@@ -564,8 +564,12 @@ struct isspa_engine {
         a.done_ptr = d_done;
         a.status = status;
         a.ov_epoch = ov_epoch;
+        a.host_pos = host_out[0];
+        a.host_vel = host_out[1];
+        a.host_force = host_out[2];
         return a;
     }
+    float4 *host_out[3] = {nullptr, nullptr, nullptr};  // set while isspa_step_host enqueues its step
 
     IntegratorArgs integrator_args() const {
         IntegratorArgs a{};
@@ -847,26 +851,34 @@ struct isspa_engine {
         ck(e);
         return ex;
     }
-    // isspa_step_host with mapped buffers: copy-in kernel, step and copy-out
-    // kernel captured as one graph per set of buffer device addresses (the
-    // last few sets kept).  The addresses are resolved through the buffer
+    // isspa_step_host with mapped buffers: copy-in kernel and step, whose update
+    // also writes the output buffers, captured as one graph per set of buffer
+    // device addresses (the last few sets kept).  The addresses are resolved through the buffer
     // registry on every call, so a graph is only launched for live buffers.
     struct HostStepGraph {
         const void *key[5];
         cudaGraphExec_t exec;
     };
     std::vector<HostStepGraph> host_graphs;
-    cudaGraphExec_t host_step_graph(const void *const key[5], const Copy3Args &in, bool has_in, const Copy3Args &out,
-                                    bool has_out) {
+    void enqueue_host_step(const Copy3Args &in, bool has_in, float4 *const out[3]) {
+        if (has_in) launch_copy3(in, stream);
+        std::copy(out, out + 3, host_out);
+        try {
+            enqueue_step_forked();
+        } catch (...) {
+            std::fill(host_out, host_out + 3, nullptr);
+            throw;
+        }
+        std::fill(host_out, host_out + 3, nullptr);
+    }
+    cudaGraphExec_t host_step_graph(const void *const key[5], const Copy3Args &in, bool has_in, float4 *const out[3]) {
         for (const HostStepGraph &h : host_graphs)
             if (std::equal(h.key, h.key + 5, key)) return h.exec;
         prepare_merged();
         cudaGraph_t g = nullptr;
         ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         try {
-            if (has_in) launch_copy3(in, stream);
-            enqueue_step_forked();
-            if (has_out) launch_copy3(out, stream);
+            enqueue_host_step(in, has_in, out);
         } catch (...) {
             cudaStreamEndCapture(stream, &g);
             if (g) cudaGraphDestroy(g);
@@ -2206,9 +2218,9 @@ int isspa_step_host(isspa_engine *e, const float *pin, const float *vin, float *
     int rc = guard(e);
     if (rc) return rc;
     const size_t b = sizeof(float4) * e->n_atoms;
-    // Buffers that all come from isspa_host_alloc are read and written by two
-    // small kernels around the step (the GPU reaches page-locked host memory
-    // directly); anything else goes through one copy per buffer.
+    // Buffers that all come from isspa_host_alloc are read by a small kernel
+    // ahead of the step and written by its update (the GPU reaches page-locked
+    // host memory directly); anything else goes through one copy per buffer.
     const auto *dpin = static_cast<const float4 *>(host_mapped(pin, b));
     const auto *dvin = static_cast<const float4 *>(host_mapped(vin, b));
     auto *dpout = static_cast<float4 *>(host_mapped(pout, b));
@@ -2218,16 +2230,14 @@ int isspa_step_host(isspa_engine *e, const float *pin, const float *vin, float *
     return run_guarded([&] {
         if (direct) {
             const Copy3Args in{{dpin, dvin, nullptr}, {e->pos, e->vel, nullptr}, e->n_atoms};
-            const Copy3Args out{{pout ? e->pos : nullptr, vout ? e->vel : nullptr, fout ? e->force_out : nullptr},
-                                {dpout, dvout, dfout}, e->n_atoms};
-            const bool has_in = pin || vin, has_out = pout || vout || fout;
+            float4 *const out[3] = {dpout, dvout, dfout};
+            const bool has_in = pin || vin;
             if (e->opt.use_graph) {
                 const void *key[5] = {dpin, dvin, dpout, dvout, dfout};
-                ck(cudaGraphLaunch(e->host_step_graph(key, in, has_in, out, has_out), e->stream));
+                ck(cudaGraphLaunch(e->host_step_graph(key, in, has_in, out), e->stream));
             } else {
-                if (has_in) launch_copy3(in, e->stream);
-                e->run_steps(1);
-                if (has_out) launch_copy3(out, e->stream);
+                e->prepare_merged();
+                e->enqueue_host_step(in, has_in, out);
             }
             ck(cudaGetLastError());
         } else {

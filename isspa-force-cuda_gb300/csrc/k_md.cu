@@ -241,6 +241,7 @@ void launch_cell_index(const float4 *pos, int off, int n, float rc, int3 nc, int
 }
 
 __global__ void copy3_kernel(Copy3Args a) {
+    pdl_trigger();  // (the step's first kernel waits for this one before it reads a position)
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
 #pragma unroll

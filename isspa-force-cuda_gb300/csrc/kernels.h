@@ -165,6 +165,8 @@ struct LeapfrogArgs {
     unsigned int *done_ptr;    // block-completion counter (self-resetting)
     int *status;
     unsigned int *ov_epoch;    // advanced with the step counter (the field-tile stamps' base)
+    // page-locked host buffers that the update also writes (nullptr: not asked for)
+    float4 *host_pos, *host_vel, *host_force;
 };
 
 // Fused integrator: the bonded terms, the umbrella restraint and leapfrog of a

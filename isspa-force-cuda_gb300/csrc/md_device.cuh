@@ -490,6 +490,7 @@ __device__ __forceinline__ void leapfrog_finish(const LeapfrogArgs &a, int i, co
     acc[1] = 0ull;
     acc[2] = 0ull;
     a.force_out[i] = make_float4(fx, fy, fz, 0.0f);
+    if (a.host_force) a.host_force[i] = make_float4(fx, fy, fz, 0.0f);
     float4 v = q.v, x = q.x;
     if (q.hit) {
         v.x = fmaf(q.gx, q.sd, __fmul_rn(fx, q.k));
@@ -512,6 +513,8 @@ __device__ __forceinline__ void leapfrog_finish(const LeapfrogArgs &a, int i, co
         atomicOr(a.status, kStatusNonFinite);
     a.vel[i] = v;
     a.pos[i] = x;
+    if (a.host_vel) a.host_vel[i] = v;
+    if (a.host_pos) a.host_pos[i] = x;
 }
 __device__ __forceinline__ void leapfrog_atom(const LeapfrogArgs &a, int i, uint32_t step, const long long *extra) {
     leapfrog_finish(a, i, leapfrog_prepare(a, i, step), extra);
