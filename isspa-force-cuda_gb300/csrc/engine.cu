@@ -321,26 +321,29 @@ struct isspa_engine {
 
     long long nonbond_items_for(long long J) const {
         long long n = 0;
-        for (const WinDev &d : win_h) n += ((d.n_atoms + 127) / 128) * ((d.n_atoms + J - 1) / J);
+        for (const WinDev &d : win_h) n += ((d.n_atoms + kNbRows - 1) / kNbRows) * ((d.n_atoms + J - 1) / J);
         return n;
     }
     // The longest partner stretch (fewest stage set-ups and atomics) whose
-    // items still fill two waves of resident blocks; 128 when none does.
+    // items still fill four waves of resident blocks; 128 when none does.  Us per
+    // solvent-free step with two / four / eight waves: 4400 atoms 35.2 / 34.8 /
+    // 34.8, 6600 67.2 / 66.3 / 68.1, 8800 109.3 / 107.6 / 108.0.
     int default_nonbond_chunk() const {
         const long long slots = (long long)n_sms * std::max(1, nonbond_blocks_per_sm(n_lj_types));
         for (int J : {4096, 2048, 1024, 768, 512, 384, 256})
-            if (nonbond_items_for(J) >= 2 * slots) return J;
+            if (nonbond_items_for(J) >= 4 * slots) return J;
         return 128;
     }
     // Nonbond work items, partner-chunk-major: blocks that run together add
-    // into different receiving tiles.  Per-stage sums start at multiples of
-    // 128 partners from the window's first atom, so J moves no result.
+    // into different receiving tiles.  J is a multiple of 128 partners, and the
+    // FP32 sums are those of 32 partners, so J moves no result.
+    static constexpr int kNbRows = 32;  // receiving atoms per item
     void nonbond_items(int J, std::vector<int4> &items, std::vector<int> &nj) const {
         for (int w : order) {
             const WinDev &d = win_h[w];
             for (int j = 0; j < d.n_atoms; j += J)
-                for (int a = 0; a < d.n_atoms; a += 128) {
-                    items.push_back(make_int4(w, d.atom_off + a, std::min(128, d.n_atoms - a), d.atom_off + j));
+                for (int a = 0; a < d.n_atoms; a += kNbRows) {
+                    items.push_back(make_int4(w, d.atom_off + a, std::min(kNbRows, d.n_atoms - a), d.atom_off + j));
                     nj.push_back(std::min(J, d.n_atoms - j));
                 }
         }

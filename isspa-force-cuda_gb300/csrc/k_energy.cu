@@ -17,7 +17,7 @@
 //            v(t+dt/2) = v(t-dt/2) + F(t) dt/m (leapfrog_cuda.cu:57-60), and
 //            the umbrella k/2 (d - x0)^2 (us_force_cuda.cu:14-48).
 // The virial is sum r . F over the same terms.  Pair energies are evaluated
-// in FP32 with the force kernel's geometry and summed per stage of 128
+// in FP32 with the force kernel's geometry and summed per group of 32
 // partners in FP32, then in FP64; bonded terms are FP64 throughout (as their
 // forces); every cross-thread reduction is FP64 (warp shuffles, then one
 // atomicAdd per warp or block and component).
@@ -29,7 +29,7 @@
 namespace isspa {
 namespace {
 
-constexpr int kEnThreads = 128;  // = the nonbond work items' atoms per item
+constexpr int kEnThreads = 128;  // four warps: the nonbond work items' 32 atoms, a quarter of each stage's partners
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -60,8 +60,8 @@ __device__ __forceinline__ void window_add(double *energy, int w, const double (
     }
 }
 
-// Same work items and partner order as the nonbond force kernel; all atoms
-// of an item belong to one window.  Ordered pairs, halved at the end.
+// Same work items as the nonbond force kernel, and its groups of 32 partners;
+// all atoms of an item belong to one window.  Ordered pairs, halved at the end.
 __global__ void __launch_bounds__(kEnThreads) nonbond_energy_kernel(NonbondArgs a, double *energy) {
     __shared__ float4 s_x[kEnThreads];
     __shared__ float4 s_c[kEnThreads];  // rmax_j, (2 rmax_j)^2, 4 rmax_j, (1-1/ep)/(24 rmax_j^4)
@@ -72,8 +72,9 @@ __global__ void __launch_bounds__(kEnThreads) nonbond_energy_kernel(NonbondArgs 
     const int nj = a.items_nj[blockIdx.x];
     const WinDev W = a.win[item.x];
     const int t = threadIdx.x;
-    const bool active = t < item.z;
-    const int i = item.y + (active ? t : 0);
+    const int lane = t & 31, wp = t >> 5;
+    const bool active = lane < item.z;
+    const int i = item.y + (active ? lane : 0);
     const float4 xi = a.pos[i];
     const int trow = a.atype[i].x * a.n_lj_types;
     const float L = W.box, h = W.hbox;
@@ -83,8 +84,6 @@ __global__ void __launch_bounds__(kEnThreads) nonbond_energy_kernel(NonbondArgs 
 
     int cur = a.excl_start[i];
     const int end = a.excl_start[i + 1];
-    while (cur < end && a.excl[cur] < item.w) ++cur;
-    int next_ex = cur < end ? a.excl[cur] : INT_MAX;
 
     double elj = 0.0, ecoul = 0.0, ecorr = 0.0, vir = 0.0;
     for (int j0 = 0; j0 < nj; j0 += kEnThreads) {
@@ -103,7 +102,10 @@ __global__ void __launch_bounds__(kEnThreads) nonbond_energy_kernel(NonbondArgs 
             s_t[t] = ty.x;
         }
         __syncthreads();
-        for (int k = 0; k < jn; ++k) {
+        const int k0 = 32 * wp;
+        while (cur < end && a.excl[cur] < item.w + j0 + k0) ++cur;
+        int next_ex = cur < end ? a.excl[cur] : INT_MAX;
+        for (int k = k0; k < min(k0 + 32, jn); ++k) {
             const int j = item.w + j0 + k;
             const bool ex = j == next_ex;
             if (ex) {
@@ -151,11 +153,10 @@ __global__ void __launch_bounds__(kEnThreads) nonbond_energy_kernel(NonbondArgs 
         vir += vr;
     }
     double v[4] = {active ? elj : 0.0, active ? ecoul : 0.0, active ? ecorr : 0.0, active ? vir : 0.0};
-    const int lane = t & 31, wid = t >> 5;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         v[k] = warp_sum(v[k]);
-        if (lane == 0) s_red[k][wid] = v[k];
+        if (lane == 0) s_red[k][wp] = v[k];
     }
     __syncthreads();
     if (t == 0) {

@@ -908,7 +908,7 @@ struct MergedSmem {
     union {
         FusedSmem<S> tile;
         struct {
-            NonbondSmem nb[FieldShape<S>::kThreads / kNbThreads];
+            NonbondSmem<kNbThreads> nb[FieldShape<S>::kThreads / kNbThreads];
             float2 ab[kMergedMaxAB];
         };
         struct {
@@ -987,9 +987,9 @@ __global__ void __launch_bounds__(FieldShape<S>::kThreads) merged_step_kernel(Me
         if (const int r = b % m.n_copies) g.facc = m.copies + 3 * (long long)(r - 1) * m.lf.n_atoms;
         field_force_tile<S, false, TS>(f, g, b, sm.tile);
     } else if ((b -= m.field.n_tiles) < m.nonbond.n_items) {
-        // a block's groups of 128 threads take the stages of its item, which
-        // are summed into fixed point stage by stage in any case
-        for (int k = threadIdx.x; k < m.nonbond.n_lj_types * m.nonbond.n_lj_types; k += kT) sm.ab[k] = m.nonbond.ljab[k];
+        // a block's groups of 128 threads take 128 partners of its item each
+        // (the sums are folded into fixed point 32 partners at a time in any case)
+        stage_ljab(m.nonbond, sm.ab);
         const int g = threadIdx.x / kNbThreads;
         int4 item = m.nonbond.items[b];
         const int nj = min(kNbThreads, m.nonbond.items_nj[b] - g * kNbThreads);
@@ -997,8 +997,8 @@ __global__ void __launch_bounds__(FieldShape<S>::kThreads) merged_step_kernel(Me
         if (nj > 0) {
             nonbond_range<true, NB_ALL, true>(m.nonbond, item, nj, threadIdx.x % kNbThreads, sm.nb[g], sm.ab);
         } else {
-            __syncthreads();
             pdl_wait();
+            __syncthreads();
             __syncthreads();
         }
         pdl_trigger();
@@ -1148,7 +1148,7 @@ cudaError_t launch_step(const StepArgs &a, int grid, cudaStream_t s) {
 }
 
 int merged_threads(int split) { return 32 * split; }
-int merged_nonbond_partners(int split) { return 32 * split; }  // a stage of 128 per group of 128 threads
+int merged_nonbond_partners(int split) { return 32 * split; }  // 128 per group of 128 threads
 
 namespace {
 template <int S, bool TS>

@@ -17,171 +17,177 @@ namespace {
 constexpr int kNbThreads = 128;
 constexpr int kNbMaxAB = 4096;  // LJ type pairs held in shared memory (up to 64 LJ types)
 
-// One work item: 128 receiving atoms i (one per thread) against nj partners j
-// starting at item.w, streamed through shared memory in stages of 128.  The
-// per-stage FP32 sums are folded into fixed point per stage, and stages start
-// at multiples of 128 partners from the window's first atom whatever the item
-// length, so the forces do not depend on the partners per item (an autotuned
-// shape).  Exclusions and the self pair are found per stage as a 128-bit mask
-// from the atom's sorted exclusion list; a group of 32 partners that no lane
-// of the warp excludes runs without per-pair checks.  SMEM_AB: the LJ (A, B)
-// table of every ordered type pair sits in shared memory (dynamic, nt^2
-// float2) instead of a global gather per pair.  ALL: every term on (mask 7).
+// One work item: 32 receiving atoms i (one per lane) against nj partners j
+// starting at item.w (a multiple of 128 partners from the window's first atom).
+// The partners are staged in shared memory, and the four warps take groups of 32
+// of them in turn.  A group's FP32 sums are folded into fixed point, so the
+// forces depend neither on the partners per item (an autotuned shape) nor on
+// which warp took a group.  Exclusions and the self pair are a 32-bit mask per
+// group from the atom's sorted exclusion list; a group that no lane excludes
+// runs without per-pair checks.
 //
-// The item's thread t of kNbThreads; every thread of the block calls this, with
-// two barriers per stage.  WAIT: a programmatic dependent that waits for the
-// kernel before it here, once everything that does not move between steps
-// (types, exclusions, parameters) has been read.
+// A lane used to take all 128 partners of a stage, and a small system waits for
+// that chain.  Four warps on one row tile cut it to 32 pairs: a solvent-free step
+// of 264 / 1100 / 2200 / 3300 atoms takes 9.5 / 10.0 / 15.9 / 23.8 us, with a
+// thread per row 12.4 / 13.1 / 18.7 / 35.3.  From about 4400 atoms on the pass is
+// bound by issue (83 % of the slots, 43 instructions per 32 pairs, most of them
+// the image's compare and select and the pair's multiplies), and the pair counts:
+// every term shares q_i q_j, the staged constants fold the correction into two
+// multiply-adds and the LJ table holds 12 A and -6 B (4400 / 8800 atoms: 34.8 /
+// 107.6 us, before 36.7 / 111.4).
+// SMEM_AB: that table of every ordered type pair sits in shared memory
+// (dynamic, nt^2 float2) instead of a global gather per pair.  ALL: every term
+// on (mask 7).
+//
+// t: the thread's index in the item (of kNbThreads); every thread of the block
+// calls this, with two barriers per stage.  WAIT: a programmatic dependent that
+// waits for the kernel before it here, once everything that does not move
+// between steps (types, exclusions, parameters) has been read; one stage only.
+template <int STAGE>  // partners staged at a time
 struct NonbondSmem {
-    float4 x[kNbThreads];
-    float4 c[kNbThreads];  // rmax_j, (2 rmax_j)^2, 8 rmax_j, (1-1/ep)/(24 rmax_j^4)
-    int t[kNbThreads];
+    static constexpr int kNbStage = STAGE;
+    float4 x[kNbStage];
+    // (2 rmax_j)^2, 8 rmax_j k, -3 k with k = (1-1/ep)/(24 rmax_j^4); byte offset of
+    // the LJ type in a row of the table
+    float4 c[kNbStage];
+    long long fix[3][kNbThreads];
 };
-template <bool SMEM_AB, bool ALL, bool WAIT = false>
-__device__ __forceinline__ void nonbond_range(const NonbondArgs &a, int4 item, int nj, int t, NonbondSmem &sm,
+template <bool SMEM_AB, bool ALL, bool WAIT = false, class Smem>
+__device__ __forceinline__ void nonbond_range(const NonbondArgs &a, int4 item, int nj, int t, Smem &sm,
                                               const float2 *s_ab) {
-    float4 *const s_x = sm.x, *const s_c = sm.c;
-    int *const s_t = sm.t;
+    constexpr int kNbStage = Smem::kNbStage;
     const WinDev W = a.win[item.x];
-    const bool active = t < item.z;
-    const int i = item.y + (active ? t : 0);
-    float4 xi;
-    if (!WAIT) xi = a.pos[i];
+    const int lane = t & 31, wp = t >> 5;
+    const bool active = lane < item.z;
+    const int i = item.y + (active ? lane : 0);
     const int nt = a.n_lj_types;
-    const int trow = a.atype[i].x * nt;
+    const char *const row = reinterpret_cast<const char *>((SMEM_AB ? s_ab : a.ljab) + a.atype[i].x * nt);
     const float L = W.box, h = W.hbox;
     const int terms = ALL ? 7 : a.terms;
     const float epf = 1.0f - 1.0f / kEp;
-    const float kfar = -2.0f * epf / 3.0f;
+    const float kfar = -2.0f * epf / 3.0f, kfar1 = 1.0f + kfar;
 
-    // exclusion cursor: first entry >= first partner of this item; the list
-    // is sorted, so an item outside [first, last] entry needs no walk
     const int end = a.excl_start[i + 1];
     int cur = a.excl_start[i];
-    if (cur < end) {
-        if (a.excl[end - 1] < item.w || a.excl[cur] >= item.w + nj) cur = end;
-        else
-            while (cur < end && a.excl[cur] < item.w) ++cur;
-    }
-
-    long long fxa = 0, fya = 0, fza = 0;  // per-stage partial sums in fixed point
-    for (int j0 = 0; j0 < nj; j0 += kNbThreads) {
-        const int jn = min(kNbThreads, nj - j0);
-        const int jb = item.w + j0;  // first partner of the stage
-        // exclusion / self bits of this stage's 128 partners
-        unsigned m[4] = {0u, 0u, 0u, 0u};  // register-resident: constant indices only
-        auto set_bit = [&](int b) {
-            const unsigned bit = 1u << (b & 31);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) m[q] |= (b >> 5) == q ? bit : 0u;
-        };
+    // exclusion / self bits of the 32 partners from jb on (groups in increasing order)
+    auto group_mask = [&](int jb, int kn) {
+        while (cur < end && a.excl[cur] < jb) ++cur;
+        unsigned m = 0u;
         for (; cur < end; ++cur) {
             const int b = a.excl[cur] - jb;
-            if (b >= kNbThreads || j0 + b >= nj) break;
-            set_bit(b);
+            if (b >= kn) break;
+            m |= 1u << b;
         }
-        if (i - jb >= 0 && i - jb < kNbThreads) set_bit(i - jb);
-        float ax = 0.f, ay = 0.f, az = 0.f;
-        __syncthreads();
-        if (t < jn) {
-            const int2 ty = a.atype[jb + t];
+        if (i - jb >= 0 && i - jb < kn) m |= 1u << (i - jb);
+        return m;
+    };
+    unsigned m0 = 0u;
+    if (32 * wp < nj) m0 = group_mask(item.w + 32 * wp, min(32, nj - 32 * wp));
+    float4 xi;
+    if (!WAIT) xi = a.pos[i];
+
+    long long f[3] = {0, 0, 0};
+    for (int j0 = 0; j0 < nj; j0 += kNbStage) {
+        const int jn = min(kNbStage, nj - j0);
+        if (j0 > 0) __syncthreads();  // the previous stage has been read
+        for (int k = t; k < jn; k += kNbThreads) {
+            const int2 ty = a.atype[item.w + j0 + k];
             const float rm = __ldg(a.rmax + ty.y);
             const float two = 2.0f * rm;
             const float r2 = rm * rm;
-            s_c[t] = make_float4(rm, __fmul_rn(two, two), 8.0f * rm, epf / (24.0f * r2 * r2));
-            s_t[t] = ty.x;
+            const float kc = epf / (24.0f * r2 * r2);
+            sm.c[k] = make_float4(__fmul_rn(two, two), 8.0f * rm * kc, -3.0f * kc, __int_as_float((int)sizeof(float2) * ty.x));
         }
-        if (WAIT && j0 == 0) {
+        if (WAIT) {
             pdl_wait();
             xi = a.pos[i];
         }
-        if (t < jn) s_x[t] = a.pos[jb + t];
+        for (int k = t; k < jn; k += kNbThreads) sm.x[k] = a.pos[item.w + j0 + k];
         __syncthreads();
-        // the pair (i, staged partner k); EX: excluded (IS-SPA correction
-        // only).  MASKED: the exclusion bit and the self pair are applied by
-        // selects instead of branches (the self pair gets d2 = 1 and adds
-        // nothing), so a group with exclusions keeps an unrolled loop; the
-        // values are those of the branching form.
-        auto pair_t = [&](int k, bool ex, bool self, auto masked) {
-            constexpr bool MASKED = decltype(masked)::value;
-            const float4 xj = s_x[k];
-            const float rx = mimg(xi.x - xj.x, L, h);
-            const float ry = mimg(xi.y - xj.y, L, h);
-            const float rz = mimg(xi.z - xj.z, L, h);
-            const float d2 = MASKED && self ? 1.0f : dist2f(rx, ry, rz);
-            const float ri = rsqrtf(d2);
-            const float ri2 = ri * ri;
-            const float qq = xi.w * xj.w;
-            float fs = 0.0f;
-            if (terms & 4) {  // IS-SPA long-range dielectric correction (:141-147)
-                const float4 c = s_c[k];
-                fs = d2 > c.y ? kfar * qq * ri2 * ri : -qq * c.w * (c.z - 3.0f * d2 * ri);
-            }
-            if (MASKED || !ex) {
-                float fp = fs;
-                if (terms & 1) {  // LJ (:131-132)
-                    const float2 ab = SMEM_AB ? s_ab[trow + s_t[k]] : __ldg(a.ljab + trow + s_t[k]);
-                    const float r6 = ri2 * ri2 * ri2;
-                    fp += r6 * fmaf(12.0f * ab.x, r6, -6.0f * ab.y) * ri2;
+        for (int k0 = 32 * wp; k0 < jn; k0 += kNbThreads) {
+            const int kn = min(32, jn - k0), jb = item.w + j0 + k0;
+            const unsigned m = j0 + k0 == 32 * wp ? m0 : group_mask(jb, kn);
+            float ax = 0.f, ay = 0.f, az = 0.f;
+            // the pair (i, staged partner k0 + k).  MASKED: an excluded pair keeps
+            // the IS-SPA correction only, the self pair gets d2 = 1 and adds
+            // nothing, both by selects, so that the loop stays unrolled
+            auto pair = [&](int k, auto masked) {
+                constexpr bool MASKED = decltype(masked)::value;
+                const bool bit = MASKED && ((m >> k) & 1u);
+                const bool self = MASKED && jb + k == i;
+                const float4 xj = sm.x[k0 + k], c = sm.c[k0 + k];
+                const float rx = mimg(xi.x - xj.x, L, h);
+                const float ry = mimg(xi.y - xj.y, L, h);
+                const float rz = mimg(xi.z - xj.z, L, h);
+                const float d2 = self ? 1.0f : dist2f(rx, ry, rz);
+                const float ri = rsqrtf(d2);
+                const float ri2 = ri * ri;
+                const float qq = xi.w * xj.w;
+                const float tq = qq * (ri2 * ri);            // Coulomb (:136)
+                const float g = fmaf(c.z, d2 * ri, c.y);     // near correction over -q q (:141-147)
+                const float2 ab = *reinterpret_cast<const float2 *>(row + __float_as_int(c.w));
+                const float r6 = ri2 * ri2 * ri2;
+                float lj = r6 * fmaf(SMEM_AB ? ab.x : 12.0f * ab.x, r6, SMEM_AB ? ab.y : -6.0f * ab.y);  // (:131-132)
+                float fs;
+                if (ALL) {
+                    const float t0 = bit ? 0.0f : tq, kf = bit ? kfar : kfar1;
+                    lj = bit ? 0.0f : lj;
+                    fs = fmaf(lj, ri2, d2 > c.x ? tq * kf : fmaf(-qq, g, t0));
+                } else {
+                    fs = (terms & 2) && !bit ? tq : 0.0f;
+                    if (terms & 4) fs += d2 > c.x ? kfar * tq : -qq * g;
+                    if ((terms & 1) && !bit) fs = fmaf(lj, ri2, fs);
                 }
-                if (terms & 2) fp += qq * ri2 * ri;  // Coulomb (:136)
-                fs = MASKED && ex ? fs : fp;
-            }
-            if (MASKED) fs = self ? 0.0f : fs;
-            ax = fmaf(fs, rx, ax);
-            ay = fmaf(fs, ry, ay);
-            az = fmaf(fs, rz, az);
-        };
-        auto pair = [&](int k, bool ex) { pair_t(k, ex, false, std::false_type{}); };
-#pragma unroll
-        for (int q = 0; q < kNbThreads / 32; ++q) {
-            const int k0 = 32 * q;
-            if (k0 >= jn) break;
-            const int kn = min(32, jn - k0);
-            const unsigned mq = m[q];
-            if (__any_sync(0xffffffffu, mq != 0u)) {
-                // exclusions or the self pair in this group: masked pairs,
-                // unrolled like the unmasked group below
-                const int self_k = i - (jb + k0);  // the self pair's k, if in this group
+                if (MASKED) fs = self ? 0.0f : fs;
+                ax = fmaf(fs, rx, ax);
+                ay = fmaf(fs, ry, ay);
+                az = fmaf(fs, rz, az);
+            };
+            if (__any_sync(0xffffffffu, m != 0u)) {
                 if (kn == 32) {
 #pragma unroll 4
-                    for (int k = 0; k < 32; ++k)
-                        pair_t(k0 + k, (mq >> k) & 1u, k == self_k, std::true_type{});
+                    for (int k = 0; k < 32; ++k) pair(k, std::true_type{});
                 } else {
 #pragma unroll 1
-                    for (int k = 0; k < kn; ++k)
-                        pair_t(k0 + k, (mq >> k) & 1u, k == self_k, std::true_type{});
+                    for (int k = 0; k < kn; ++k) pair(k, std::true_type{});
                 }
             } else if (kn == 32) {
 #pragma unroll 8
-                for (int k = 0; k < 32; ++k) pair(k0 + k, false);
+                for (int k = 0; k < 32; ++k) pair(k, std::false_type{});
             } else {
 #pragma unroll 1
-                for (int k = 0; k < kn; ++k) pair(k0 + k, false);
+                for (int k = 0; k < kn; ++k) pair(k, std::false_type{});
             }
+            if (active) check_force(a.status, ax, ay, az);
+            f[0] += to_fix(ax);
+            f[1] += to_fix(ay);
+            f[2] += to_fix(az);
         }
-        if (active) check_force(a.status, ax, ay, az);
-        fxa += to_fix(ax);
-        fya += to_fix(ay);
-        fza += to_fix(az);
     }
-    if (!active) return;
-    unsigned long long *acc = a.facc + 3 * (long long)i;
-    atomicAdd(acc + 0, (unsigned long long)fxa);
-    atomicAdd(acc + 1, (unsigned long long)fya);
-    atomicAdd(acc + 2, (unsigned long long)fza);
+    // the four warps' sums, one atomic per atom and component
+    for (int k = 0; k < 3; ++k) sm.fix[k][t] = f[k];
+    __syncthreads();
+    if (wp < 3 && active) {
+        long long v = 0;
+        for (int q = 0; q < kNbThreads / 32; ++q) v += sm.fix[wp][32 * q + lane];
+        atomicAdd(a.facc + 3 * (long long)i + wp, (unsigned long long)v);
+    }
 }
 
 template <bool SMEM_AB, bool ALL>
 __device__ __forceinline__ void nonbond_item(const NonbondArgs &a, int item_index, const float2 *s_ab) {
-    __shared__ NonbondSmem sm;
+    __shared__ NonbondSmem<kNbThreads> sm;
     nonbond_range<SMEM_AB, ALL>(a, a.items[item_index], a.items_nj[item_index], threadIdx.x, sm, s_ab);
+    __syncthreads();  // (a further item of the block reuses the buffers)
 }
 
-// Stages the LJ (A, B) table of every ordered type pair into shared memory
-// (read only after the item's first barrier).
+// Stages 12 A and -6 B of every ordered type pair into shared memory (read only
+// after the item's first barrier).
 __device__ __forceinline__ void stage_ljab(const NonbondArgs &a, float2 *s_ab) {
-    for (int k = threadIdx.x; k < a.n_lj_types * a.n_lj_types; k += blockDim.x) s_ab[k] = a.ljab[k];
+    for (int k = threadIdx.x; k < a.n_lj_types * a.n_lj_types; k += blockDim.x) {
+        const float2 ab = a.ljab[k];
+        s_ab[k] = make_float2(12.0f * ab.x, -6.0f * ab.y);
+    }
 }
 
 // Bonded terms in FP32.  Image vectors as the reference decides them
