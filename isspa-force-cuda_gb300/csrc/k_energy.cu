@@ -274,9 +274,9 @@ __global__ void state_energy_kernel(StateEnergyArgs a, double *energy) {
         const float4 vel = a.vel[i];
         const unsigned long long *acc = a.facc + 3 * (long long)i;
         // the integrator's own arithmetic for the kick (k_md.cu leapfrog_atom)
-        const float fx = (float)((double)(long long)acc[0] * kFixInv);
-        const float fy = (float)((double)(long long)acc[1] * kFixInv);
-        const float fz = (float)((double)(long long)acc[2] * kFixInv);
+        const float fx = from_fix((long long)acc[0]);
+        const float fy = from_fix((long long)acc[1]);
+        const float fz = from_fix((long long)acc[2]);
         const float m = vel.w, k = W.dt / m;
         const float px = vel.x + fx * k, py = vel.y + fy * k, pz = vel.z + fz * k;
         const double hm = 0.5 * (double)m;

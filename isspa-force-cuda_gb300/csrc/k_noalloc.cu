@@ -165,8 +165,8 @@ __global__ void noalloc_finish(const unsigned long long *facc, int n, float4 *ou
     if (status_out && i == 0) *status_out = *status;
     if (i >= n) return;
     const unsigned long long *a = facc + 3 * (long long)i;
-    out[i] = make_float4((float)((double)(long long)a[0] * kFixInv), (float)((double)(long long)a[1] * kFixInv),
-                         (float)((double)(long long)a[2] * kFixInv), 0.0f);
+    out[i] = make_float4(from_fix((long long)a[0]), from_fix((long long)a[1]),
+                         from_fix((long long)a[2]), 0.0f);
 }
 
 }  // namespace

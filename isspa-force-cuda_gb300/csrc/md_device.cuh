@@ -489,9 +489,9 @@ __device__ __forceinline__ void leapfrog_finish(const LeapfrogArgs &a, int i, co
     long long s[3] = {(long long)__ldcg(acc + 0), (long long)__ldcg(acc + 1), (long long)__ldcg(acc + 2)};
     if (extra)
         for (int k = 0; k < 3; ++k) s[k] += extra[k];
-    const float fx = (float)((double)s[0] * kFixInv);
-    const float fy = (float)((double)s[1] * kFixInv);
-    const float fz = (float)((double)s[2] * kFixInv);
+    const float fx = from_fix(s[0]);
+    const float fy = from_fix(s[1]);
+    const float fz = from_fix(s[2]);
     acc[0] = 0ull;
     acc[1] = 0ull;
     acc[2] = 0ull;
