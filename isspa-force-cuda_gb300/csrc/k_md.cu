@@ -28,10 +28,18 @@ namespace isspa {
 namespace {
 
 template <bool SMEM_AB, bool ALL>
-__global__ void __launch_bounds__(kNbThreads, 8) nonbond_kernel(NonbondArgs a) {
+__global__ void __launch_bounds__(kNbThreads, 8) nonbond_kernel(NonbondArgs a, BondedArgs b, int n_bonded) {
     extern __shared__ float2 s_ab[];
+    if ((int)blockIdx.x < n_bonded) {  // bonded terms of the same step, a thread each
+        pdl_wait();
+        pdl_trigger();
+        bonded_term(b, (long long)blockIdx.x * kNbThreads + threadIdx.x, FixAdd{b.facc, b.status});
+        return;
+    }
     if (SMEM_AB) stage_ljab(a, s_ab);
-    nonbond_item<SMEM_AB, ALL>(a, blockIdx.x, s_ab);
+    pdl_wait();
+    pdl_trigger();
+    nonbond_item<SMEM_AB, ALL>(a, blockIdx.x - n_bonded, s_ab);
 }
 
 __global__ void bonded_kernel(BondedArgs a) {
@@ -157,17 +165,23 @@ __global__ void fma_peak_kernel(float *out, int iters, float seed) {
 
 int nonbond_block_threads() { return kNbThreads; }
 
-void launch_nonbond(const NonbondArgs &a, cudaStream_t s) {
+int bonded_blocks(const BondedArgs &b, int threads) {
+    const long long n = (b.do_bonds ? b.n_bonds : 0) + (b.do_angles ? b.n_angles : 0) + (b.do_dihs ? b.n_dihs : 0);
+    return (int)((n + threads - 1) / threads);
+}
+
+void launch_nonbond(const NonbondArgs &a, cudaStream_t s, const BondedArgs &b) {
     if (a.n_items <= 0) return;
+    const int nb = bonded_blocks(b, kNbThreads), grid = nb + a.n_items;
     const int nab = a.n_lj_types * a.n_lj_types;
     const bool all = a.terms == 7;
     if (nab <= kNbMaxAB) {
         const size_t sm = sizeof(float2) * (size_t)std::max(nab, 1);
-        if (all) nonbond_kernel<true, true><<<a.n_items, kNbThreads, sm, s>>>(a);
-        else nonbond_kernel<true, false><<<a.n_items, kNbThreads, sm, s>>>(a);
+        if (all) launch_chain_smem(nonbond_kernel<true, true>, grid, kNbThreads, sm, s, a, b, nb);
+        else launch_chain_smem(nonbond_kernel<true, false>, grid, kNbThreads, sm, s, a, b, nb);
     } else {
-        if (all) nonbond_kernel<false, true><<<a.n_items, kNbThreads, 0, s>>>(a);
-        else nonbond_kernel<false, false><<<a.n_items, kNbThreads, 0, s>>>(a);
+        if (all) launch_chain(nonbond_kernel<false, true>, grid, kNbThreads, s, a, b, nb);
+        else launch_chain(nonbond_kernel<false, false>, grid, kNbThreads, s, a, b, nb);
     }
 }
 
@@ -183,10 +197,8 @@ int nonbond_blocks_per_sm(int n_lj_types) {
 }
 
 void launch_bonded(const BondedArgs &a, cudaStream_t s) {
-    long long n = (a.do_bonds ? a.n_bonds : 0) + (a.do_angles ? a.n_angles : 0) + (a.do_dihs ? a.n_dihs : 0);
-    if (n <= 0) return;
-    const int tpb = 128;
-    bonded_kernel<<<(unsigned)((n + tpb - 1) / tpb), tpb, 0, s>>>(a);
+    const int tpb = 128, blocks = bonded_blocks(a, tpb);
+    if (blocks > 0) bonded_kernel<<<blocks, tpb, 0, s>>>(a);
 }
 
 void launch_umbrella(const UmbrellaArgs &a, cudaStream_t s) {

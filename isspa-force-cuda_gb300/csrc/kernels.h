@@ -95,8 +95,10 @@ struct NbListArgs {
     const int4 *wcell;         // per window: first cell, cells per edge (1: one cell), bits of nc / box, -
     int n_atoms;               // all windows
     int n_cells;               // all windows
+    int block_cells;           // cells made by the check's last block (else by launches of their own)
     float4 *ref;               // [Ntot] positions at the last build (NaN before the first)
     int *flag;                 // 1: rebuild this step
+    unsigned int *count;       // [2] blocks done: check or update, pairs (0 at rest)
     int *stats;                // builds so far, fullest row of the last build
     int *cell_of, *cell_count, *cell_start, *cell_cursor, *cell_atoms;
     int *rows;                 // [Ntot][row_cap] partner | excluded << 31 (nullptr: counts only)
@@ -337,10 +339,17 @@ int merged_threads(int split);
 constexpr int kMergedCopies = 4;
 // prepare: only sets the kernel's shared-memory limit (before a capture)
 cudaError_t launch_merged_step(const MergedArgs &m, int split, cudaStream_t s, bool prepare);
-void launch_nonbond(const NonbondArgs &a, cudaStream_t s);
-// Cutoff mode: displacement check and (when it trips) the list rebuild; then the pairs.
-void launch_nblist_build(const NbListArgs &a, cudaStream_t s);
-void launch_nblist_pairs(const NbListArgs &a, cudaStream_t s);
+// The nonbond passes; b: bonded terms that the same launch takes along (none: {}).
+int bonded_blocks(const BondedArgs &b, int threads);
+void launch_nonbond(const NonbondArgs &a, cudaStream_t s, const BondedArgs &b = {});
+// Cutoff mode: displacement check (and, when it trips, the cells); the pairs (and
+// then the rows first); the update with the next step's check; the check and a
+// count of the rows only.
+void launch_nblist_check(const NbListArgs &a, cudaStream_t s);
+void launch_nblist_pairs(const NbListArgs &a, cudaStream_t s, const BondedArgs &b = {});
+void launch_nblist_leapfrog(const LeapfrogArgs &f, const NbListArgs &a, cudaStream_t s);
+bool nblist_block_cells(int n_cells);
+void launch_nblist_count(const NbListArgs &a, cudaStream_t s);
 void launch_bonded(const BondedArgs &a, cudaStream_t s);
 void launch_umbrella(const UmbrellaArgs &a, cudaStream_t s);
 void launch_leapfrog(const LeapfrogArgs &a, cudaStream_t s);
