@@ -328,31 +328,45 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, F
     // registers live across a group.
     auto accum = [&](int k, float rx, float ry, float rz, float c) {
         const float d2 = dist2f(rx, ry, rz);
-        if (d2 <= rm2) {
-            const float ri = rsqrtf(d2);
-            ++n;
+        // the in-range part behind a vote of the warp, its lanes predicated: as a
+        // branch of each lane it split the warp for one pair in six (1100 atoms:
+        // 89 -> 87 us per launch, twelve windows of 44 to 1100 atoms 390 -> 322)
+        const bool in = d2 <= rm2;
+        if (!__any_sync(0xffffffffu, in)) {
+            fx = fmaf(-c, rx, fx);
+            fy = fmaf(-c, ry, fy);
+            fz = fmaf(-c, rz, fz);
+            return;
+        }
+        if (in) {
             ex = fmaf(-c, rx, ex);
             ey = fmaf(-c, ry, ey);
             ez = fmaf(-c, rz, ez);
-            const float dist = one_grid ? density_table_dist(d2, ri) : __fsqrt_rn(d2);
-            const int bin = (int)__fmul_rn(__fsub_rn(dist, g_r0), g_inv);
-            if (bin < 0) {
-                w = 0.0f;
-            } else if (bin < nb) {
-                const int row = TMA ? __ldg(&a.atype[W.atom_off + jbase + k].y) * nb : s_row[k];
-                const float4 t = table_entry<TS>(a.gtab + row + bin);
-                const float fg = (dist - fmaf((float)bin, g_dr, g_r0)) * g_inv;
-                w *= fmaf(fg, t.y - t.x, t.x);
-                const float fe = (dist - fmaf((float)bin, e_dr, e_r0)) * e_inv;
-                const float et = fmaf(fe, t.w - t.z, t.z) * ri;
-                ex = fmaf(et, rx, ex);
-                ey = fmaf(et, ry, ey);
-                ez = fmaf(et, rz, ez);
-            }
+            ++n;
         } else {
             fx = fmaf(-c, rx, fx);
             fy = fmaf(-c, ry, fy);
             fz = fmaf(-c, rz, fz);
+        }
+        const float ri = rsqrtf(d2);
+        const float dist = one_grid ? density_table_dist(d2, ri) : __fsqrt_rn(d2);
+        const int bin = (int)__fmul_rn(__fsub_rn(dist, g_r0), g_inv);
+        if (in && bin < 0) w = 0.0f;
+        const bool ok = in && bin >= 0 && bin < nb;
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ok) {
+            const int row = TMA ? __ldg(&a.atype[W.atom_off + jbase + k].y) * nb : s_row[k];
+            t = table_entry<TS>(a.gtab + row + bin);
+        }
+        const float fg = (dist - fmaf((float)bin, g_dr, g_r0)) * g_inv;
+        const float wn = w * fmaf(fg, t.y - t.x, t.x);
+        const float fe = (dist - fmaf((float)bin, e_dr, e_r0)) * e_inv;
+        const float et = fmaf(fe, t.w - t.z, t.z) * ri;
+        if (ok) {
+            w = wn;
+            ex = fmaf(et, rx, ex);
+            ey = fmaf(et, ry, ey);
+            ez = fmaf(et, rz, ez);
         }
     };
 
@@ -564,14 +578,18 @@ struct ForceShape {
 // image) and d2 = |r|^2: the multipole terms (:274-289, with the CDD term
 // (:306-312) folded into the record D) into q per unit -q_i vtot_i, the
 // tabulated mean LJ force (:291-305) into l per unit -vtot_i.  rm2 and frow
-// belong to the atom's type; FAR: the point is known to lie outside rmax.
+// belong to the atom's type; FAR: the point is known to lie outside rmax; WARP:
+// every lane of the warp is here, and the tabulated part sits behind a vote with
+// its lanes predicated (as a branch of each lane it split the warp for one pair
+// in seven: with the root from ri 150 -> 137 us per launch at 1100 atoms, 750 ->
+// 702 for twelve windows of 44 to 1100).
 // Horner form in g = (E^.r) / r^2 with r^-3 factored out of the whole: four FP32
 // operations fewer than term by term (16 384-atom kind of window, voted loop:
 // 8800 atoms nMC 100 12.63 -> 12.22 ms per launch; 12 windows of 44 to 1100 atoms
 // 542 -> 534 us).  Packing two points into f32x2 instructions was tried again with
 // it and costs more: a packed FMA of three distinct operands takes 4.1 cycles of
 // register reads per SM quarter against 2.3 for two scalar ones.
-template <bool LJ, bool FAR, bool TS = false>
+template <bool LJ, bool FAR, bool TS = false, bool WARP = false>
 __device__ __forceinline__ void point_force(const float4 *R, float rx, float ry, float rz, float d2, float rm2,
                                             int frow, const ForceArgs &a, float &qx, float &qy, float &qz,
                                             float &lx, float &ly, float &lz) {
@@ -591,13 +609,16 @@ __device__ __forceinline__ void point_force(const float4 *R, float rx, float ry,
     qx = fmaf(ri3, fmaf(Z, rx, fmaf(-Y, E.x, -D.x)), qx);
     qy = fmaf(ri3, fmaf(Z, ry, fmaf(-Y, E.y, -D.y)), qy);
     qz = fmaf(ri3, fmaf(Z, rz, fmaf(-Y, E.z, -D.z)), qz);
-    if (LJ && inside) {
-        const float dist = __fsqrt_rn(d2);
+    if (!LJ || FAR) return;
+    if (WARP ? __any_sync(0xffffffffu, inside) : inside) {
+        const float dist = pair_dist(d2, ri);
         const int bin = (int)__fmaf_rn(__fsub_rn(dist, a.f_r0), a.f_inv, 0.5f);
-        if (bin >= 0 && bin < a.n_f) {
-            const float2 tv = table_entry<TS>(a.ftab + frow + bin);
-            const float fr = (dist - fmaf((float)bin, a.f_dr, a.f_r0)) * a.f_inv;
-            const float fv = fmaf(fr, tv.y - tv.x, tv.x) * R[0].w * ri;
+        const bool ok = inside && bin >= 0 && bin < a.n_f;
+        float2 tv = make_float2(0.0f, 0.0f);
+        if (ok) tv = table_entry<TS>(a.ftab + frow + bin);
+        const float fr = (dist - fmaf((float)bin, a.f_dr, a.f_r0)) * a.f_inv;
+        const float fv = fmaf(fr, tv.y - tv.x, tv.x) * R[0].w * ri;
+        if (ok) {
             lx = fmaf(fv, rx, lx);
             ly = fmaf(fv, ry, ly);
             lz = fmaf(fv, rz, lz);
@@ -664,7 +685,7 @@ __device__ __forceinline__ void force_item(const ForceArgs &a, int item_index) {
         // the pair (staged point k, receiving atom u) after its geometry; FAR:
         // the point is known to lie outside rmax of the atom's type
         auto pair = [&](int k, int u, float rx, float ry, float rz, float d2, auto far) {
-            point_force<LJ, decltype(far)::value>(s_p[k].q, rx, ry, rz, d2, rm2[u], frow[u], a, qx[u], qy[u], qz[u],
+            point_force<LJ, decltype(far)::value, false, true>(s_p[k].q, rx, ry, rz, d2, rm2[u], frow[u], a, qx[u], qy[u], qz[u],
                                                   lx[u], ly[u], lz[u]);
         };
         int k = 0;
