@@ -117,9 +117,9 @@ typedef struct isspa_engine_options {
     int field_vote;      /* 1: the field pass walks its atoms in groups of four with one
                             warp vote on "any inside rmax" per group (same results);
                             0 => per-pair branches */
-    int force_vote;      /* 1: the force pass (one atom per thread) takes its points in
-                            groups of four with one warp vote per group (same results);
-                            0 => per-pair branches */
+    int force_vote;      /* 0 or 1, reported back; the force pass (one atom per thread)
+                            takes its points in groups of four with one warp vote per
+                            group either way */
     int integrator;      /* how isspa_step runs a step: 1 = bonded, umbrella and leapfrog
                             kernels (bonded, umbrella and nonbond on branches concurrent
                             with the IS-SPA pass);

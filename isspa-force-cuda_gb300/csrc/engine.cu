@@ -99,7 +99,7 @@ struct isspa_engine {
     size_t tile_flag_cap = 0;
     int *tile_base = nullptr;           // per window: its first field tile
     unsigned int *ov_epoch = nullptr;   // stamp of the current pass - 1 (advanced with the step counter)
-    int force_vote = 0;  // force pass in warp-voted groups of four points (1 atom per thread)
+    int force_vote = 0;  // option as given (the force pass always takes voted groups of four points)
     int force_apt = 1;  // receiving atoms per force-kernel thread (1 or 2)
     // step integrator: 1 = bonded, umbrella and leapfrog kernels (bonded and
     // umbrella on the forked branch), 2 = one fused cooperative kernel
@@ -228,16 +228,7 @@ struct isspa_engine {
     // Grids of equal-work blocks should fill whole waves of resident blocks:
     // the last, partial wave idles the remaining SMs.
     int default_field_split() const {
-        int S = 4;
-        double best = -1.0;
-        for (int cand : {1, 2, 4, 8, 16}) {
-            const double e = wave_eff(field_tiles_for(cand), (long long)n_sms * field_blocks_per_sm(cand));
-            if (e > best + 0.02) {
-                best = e;
-                S = cand;
-            }
-        }
-        return S;
+        return default_split(n_sms, [&](int S) { return field_tiles_for(S); });
     }
     int default_force_chunk() const {
         const long long slots = (long long)n_sms * std::max(1, force_blocks_per_sm(force_apt));
@@ -414,7 +405,6 @@ struct isspa_engine {
     }
     ForceArgs force_args() const {
         ForceArgs a{};
-        a.vote = force_vote;
         a.pos = pos;
         a.atype = atype;
         a.win = win;
@@ -611,7 +601,6 @@ struct isspa_engine {
         a.field.vote = 0;
         a.field.tma = 0;
         a.force = force_args();
-        a.force.vote = 0;
         a.nonbond = nonbond_args();
         a.integ = integrator_args();
         return a;
@@ -1861,14 +1850,6 @@ int isspa_autotune(isspa_engine *e, int reps, int shape[ISSPA_SHAPE_COUNT]) {
             }
         }
         e->set_force_chunk(bestC, bestT);
-        // the voted force loop on the chosen work list
-        e->force_vote = 0;
-        const float plain = time_it([&] { launch_force(e->force_args(), e->stream); });
-        e->force_vote = 1;
-        const float voted = time_it([&] { launch_force(e->force_args(), e->stream); });
-        // (in the step, among other branches' blocks, it costs about a per cent
-        // where the two time equal alone)
-        e->force_vote = voted < 0.985f * plain ? 1 : 0;
         // nonbond pass: partner stretches per item (results do not move)
         if (e->opt.nonbond_terms && e->n_nb_items > 0 && !e->cutoff) {
             int maxN = 0;

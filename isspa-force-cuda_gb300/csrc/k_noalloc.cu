@@ -189,22 +189,8 @@ extern "C" int isspa_force_noalloc(const isspa_noalloc_inputs *in_p, float *forc
     int rc = scratch_address(&base, &sms);
     if (rc) return rc;
 
-    // launch shapes: field split by wave efficiency, force chunks for >= 2 waves
-    auto eff = [](long long u, long long s) {
-        if (u <= 0 || s <= 0) return 0.0;
-        const double w = (double)u / (double)s;
-        return w / std::ceil(w);
-    };
-    int S = 4;
-    double best = -1.0;
-    for (int c : {1, 2, 4, 8, 16}) {
-        const int tp = field_points_per_block(c);
-        const double e = eff((P + tp - 1) / tp, (long long)sms * field_blocks_per_sm(c));
-        if (e > best + 0.02) {
-            best = e;
-            S = c;
-        }
-    }
+    // launch shapes: the engine's default field split, force chunks for >= 2 waves
+    const int S = default_split(sms, [&](int c) { return (P + field_points_per_block(c) - 1) / field_points_per_block(c); });
     Plan pl{};
     pl.n_atoms = in.n_atoms;
     pl.tp = field_points_per_block(S);

@@ -1,5 +1,6 @@
 // kernels.h -- argument blocks and launch wrappers of the device kernels.
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -52,7 +53,6 @@ struct ForceArgs {
     float f_r0, f_dr, f_inv;
     int terms;             // 1 multipole, 2 tabulated LJ, 4 CDD
     int atoms_per_thread;  // 1 (128-thread blocks) or 2 (64-thread blocks)
-    int vote;              // 1: points in warp-voted groups of four (same results)
     unsigned long long *facc;  // [Ntot][3]
     int *status;
     // overlap with the field pass (overlap = 1): instead of waiting for the
@@ -382,6 +382,32 @@ int nonbond_block_threads();
 // launch-shape helpers for the work-list builder
 int field_points_per_block(int split);
 int field_blocks_per_sm(int split);
+// The field pass's default split.  A pair costs less the fewer warps share a
+// tile (8800 atoms, S = 1 / 2 / 4 / 8 / 16: 6.02 / 6.59 / 6.95 / 6.76 / 6.99 ms;
+// 1100 atoms 123 / 101 / 96 / 89 / 95 us; 264 atoms 54 / 33 / 24 / 17 / 16.5), as
+// long as the tiles fill the chip: whole waves of resident blocks count, and
+// whole rounds of SMs, since a last wave's blocks run faster for being few.
+// tiles(S): a split's number of tiles.
+template <class Tiles>
+int default_split(int sms, const Tiles &tiles) {
+    auto whole = [](long long units, long long slots) {  // filled share of the rounds
+        if (units <= 0 || slots <= 0) return 0.0;
+        return (double)units / (double)((units + slots - 1) / slots * slots);
+    };
+    constexpr int kSplit[5] = {1, 2, 4, 8, 16};
+    constexpr double kCost[5] = {1.0, 1.07, 1.1, 1.1, 1.22};
+    int S = 4;
+    double best = -1.0;
+    for (int k = 0; k < 5; ++k) {
+        const long long n = tiles(kSplit[k]);
+        const double e = std::sqrt(whole(n, (long long)sms * field_blocks_per_sm(kSplit[k])) * whole(n, sms)) / kCost[k];
+        if (e > best) {
+            best = e;
+            S = kSplit[k];
+        }
+    }
+    return S;
+}
 int force_blocks_per_sm(int atoms_per_thread);
 int nonbond_blocks_per_sm(int n_lj_types);
 
