@@ -312,11 +312,13 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, F
     // geometry of the pair (point, staged atom k); true when inside rmax of
     // the owner's type (:154)
     int buf = 0, jbase = 0;  // staged buffer and first atom of the current round
-    auto geom = [&](int k, float &rx, float &ry, float &rz, float &c) {
+    const float sx = image_side(px, L, h), sy = image_side(py, L, h), sz = image_side(pz, L, h);
+    auto geom = [&](auto toward, int k, float &rx, float &ry, float &rz, float &c) {
+        constexpr bool T = decltype(toward)::value;
         const float4 xj = s_atom[TMA ? buf : 0][k];
-        rx = mimg(px - xj.x, L, h);
-        ry = mimg(py - xj.y, L, h);
-        rz = mimg(pz - xj.z, L, h);
+        rx = image<T>(px - xj.x, sx, L, h);
+        ry = image<T>(py - xj.y, sy, L, h);
+        rz = image<T>(pz - xj.z, sz, L, h);
         const float d2 = dist2f(rx, ry, rz);
         const float ri = rsqrtf(d2);
         c = (TMA ? a.e0 * xj.w : xj.w) * (ri * ri * ri);
@@ -395,6 +397,11 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, F
             stage_round(j0, jn);
             __syncthreads();
         }
+        // the warp's atoms of this round: inside the box (as the update leaves
+        // them) the image's direction is the point's
+        bool inside = true;
+        for (int q = sp + S * lane; q < jn; q += 32 * S) inside = inside && in_box(s_atom[TMA ? buf : 0][q], L);
+        auto round = [&](auto toward) {
         int k = sp;
         // Groups of kG staged atoms: one warp vote tells whether any lane has
         // any of them inside rmax.  When none does, their out-of-range Coulomb
@@ -409,7 +416,7 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, F
             float rx[kG], ry[kG], rz[kG], c[kG];
             bool any = false;
 #pragma unroll
-            for (int u = 0; u < kG; ++u) any = geom(k + u * S, rx[u], ry[u], rz[u], c[u]) || any;
+            for (int u = 0; u < kG; ++u) any = geom(toward, k + u * S, rx[u], ry[u], rz[u], c[u]) || any;
             if (__any_sync(0xffffffffu, any)) {
 #pragma unroll
                 for (int u = 0; u < kG; ++u) accum(k + u * S, rx[u], ry[u], rz[u], c[u]);
@@ -426,17 +433,20 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, F
 #pragma unroll 1
             for (; k < jn; k += S) {  // at most kG - 1 atoms
                 float rx, ry, rz, c;
-                geom(k, rx, ry, rz, c);
+                geom(toward, k, rx, ry, rz, c);
                 accum(k, rx, ry, rz, c);
             }
         } else {
 #pragma unroll 4
             for (; k < jn; k += S) {
                 float rx, ry, rz, c;
-                geom(k, rx, ry, rz, c);
+                geom(toward, k, rx, ry, rz, c);
                 accum(k, rx, ry, rz, c);
             }
         }
+        };
+        if (__all_sync(0xffffffffu, inside)) round(std::true_type{});
+        else round(std::false_type{});
     }
 
     if (S > 1) {
@@ -636,6 +646,7 @@ template <bool LJ, int A>
 __device__ __forceinline__ void force_item(const ForceArgs &a, int item_index) {
     constexpr int kT = ForceShape<A>::kThreads;
     __shared__ PointRec s_p[kForceThreads];
+    __shared__ float4 s_side[kForceThreads];  // the points' image directions
     const int4 item = a.items[item_index];
     const WinDev W = a.win[item.x];
     const int2 ch = a.chunks[item.w];
@@ -657,6 +668,12 @@ __device__ __forceinline__ void force_item(const ForceArgs &a, int item_index) {
         frow[u] = ity * nf;
         vt[u] = __ldg(a.vtot + ity);
     }
+    // atoms inside the box (as the update leaves them): the image's direction is
+    // the point's
+    bool inside = true;
+#pragma unroll
+    for (int u = 0; u < A; ++u) inside = inside && in_box(xi[u], L);
+    const bool toward = __all_sync(0xffffffffu, inside);
     // Per-stage FP32 partial sums (at most kForceThreads points) are folded into
     // per-thread fixed-point registers, so FP32 rounding never spans more than
     // one stage; one set of atomics per atom and work item.
@@ -675,7 +692,9 @@ __device__ __forceinline__ void force_item(const ForceArgs &a, int item_index) {
             const long long pg = (long long)ch.x + p0 + i;
             // through L2: in the single-kernel step the records were written
             // by other blocks of the same launch
-            s_p[i].q[0] = __ldcg(a.pts.q0 + pg);
+            const float4 P = __ldcg(a.pts.q0 + pg);
+            s_p[i].q[0] = P;
+            s_side[i] = make_float4(image_side(P.x, L, h), image_side(P.y, L, h), image_side(P.z, L, h), 0.0f);
             s_p[i].q[1] = __ldcg(a.pts.q1 + pg);
             s_p[i].q[2] = __ldcg(a.pts.q2 + pg);
             s_p[i].q[3] = __ldcg(a.pts.q3 + pg);
@@ -688,6 +707,8 @@ __device__ __forceinline__ void force_item(const ForceArgs &a, int item_index) {
             point_force<LJ, decltype(far)::value, false, true>(s_p[k].q, rx, ry, rz, d2, rm2[u], frow[u], a, qx[u], qy[u], qz[u],
                                                   lx[u], ly[u], lz[u]);
         };
+        auto stage = [&](auto toward) {
+        constexpr bool T = decltype(toward)::value;
         int k = 0;
         if (A == 1) {
             for (; k + 3 < pn; k += 4) {
@@ -696,9 +717,10 @@ __device__ __forceinline__ void force_item(const ForceArgs &a, int item_index) {
 #pragma unroll
                 for (int v = 0; v < 4; ++v) {
                     const float4 P = s_p[k + v].q[0];
-                    rx[v] = mimg(P.x - xi[0].x, L, h);
-                    ry[v] = mimg(P.y - xi[0].y, L, h);
-                    rz[v] = mimg(P.z - xi[0].z, L, h);
+                    const float4 sd = T ? s_side[k + v] : P;
+                    rx[v] = image<T>(P.x - xi[0].x, sd.x, L, h);
+                    ry[v] = image<T>(P.y - xi[0].y, sd.y, L, h);
+                    rz[v] = image<T>(P.z - xi[0].z, sd.z, L, h);
                     d2[v] = dist2f(rx[v], ry[v], rz[v]);
                     any = any || d2[v] <= rm2[0];
                 }
@@ -714,14 +736,18 @@ __device__ __forceinline__ void force_item(const ForceArgs &a, int item_index) {
 #pragma unroll 4
         for (; k < pn; ++k) {
             const float4 P = s_p[k].q[0];
+            const float4 sd = T ? s_side[k] : P;
 #pragma unroll
             for (int u = 0; u < A; ++u) {
-                const float rx = mimg(P.x - xi[u].x, L, h);
-                const float ry = mimg(P.y - xi[u].y, L, h);
-                const float rz = mimg(P.z - xi[u].z, L, h);
+                const float rx = image<T>(P.x - xi[u].x, sd.x, L, h);
+                const float ry = image<T>(P.y - xi[u].y, sd.y, L, h);
+                const float rz = image<T>(P.z - xi[u].z, sd.z, L, h);
                 pair(k, u, rx, ry, rz, dist2f(rx, ry, rz), std::false_type{});
             }
         }
+        };
+        if (toward) stage(std::true_type{});
+        else stage(std::false_type{});
 #pragma unroll
         for (int u = 0; u < A; ++u) {
             const float Fx = -vt[u] * fmaf(xi[u].w, qx[u], lx[u]);
@@ -900,7 +926,7 @@ __device__ __forceinline__ void field_force_tile(const FieldArgs &f, const Force
     tile_point_forces<true, TS>(g, W, sm.rec, tile.z, first, sm.fix());
 }
 template <int S, bool VOTE>
-__global__ void __launch_bounds__(FieldShape<S>::kThreads) field_force_kernel(FieldArgs f, ForceArgs g) {
+__global__ void __launch_bounds__(FieldShape<S>::kThreads, 1024 / FieldShape<S>::kThreads) field_force_kernel(FieldArgs f, ForceArgs g) {
     __shared__ FusedSmem<S> sm;
     static_assert(sizeof(sm.f.red) >= 3 * FieldShape<S>::kThreads * sizeof(long long), "the sums fit");
     field_force_tile<S, VOTE, false>(f, g, blockIdx.x, sm);
@@ -942,7 +968,7 @@ struct MergedSmem {
 // shared memory before the wait (a look-up inside the step is then a shared
 // load instead of an L2 round trip: the caches start the step cold).
 template <int S, bool NB_ALL, bool TS>
-__global__ void __launch_bounds__(FieldShape<S>::kThreads) merged_step_kernel(MergedArgs m) {
+__global__ void __launch_bounds__(FieldShape<S>::kThreads, 1024 / FieldShape<S>::kThreads) merged_step_kernel(MergedArgs m) {
     constexpr int kT = FieldShape<S>::kThreads;
     extern __shared__ unsigned char s_dyn[];
     MergedSmem<S> &sm = *reinterpret_cast<MergedSmem<S> *>(s_dyn);

@@ -86,6 +86,7 @@ __device__ __forceinline__ void nonbond_range(const NonbondArgs &a, int4 item, i
     float4 xi;
     if (!WAIT) xi = a.pos[i];
 
+    float sx = 0.f, sy = 0.f, sz = 0.f;
     long long f[3] = {0, 0, 0};
     for (int j0 = 0; j0 < nj; j0 += kNbStage) {
         const int jn = min(kNbStage, nj - j0);
@@ -104,21 +105,26 @@ __device__ __forceinline__ void nonbond_range(const NonbondArgs &a, int4 item, i
         }
         for (int k = t; k < jn; k += kNbThreads) sm.x[k] = a.pos[item.w + j0 + k];
         __syncthreads();
+        sx = image_side(xi.x, L, h);
+        sy = image_side(xi.y, L, h);
+        sz = image_side(xi.z, L, h);
         for (int k0 = 32 * wp; k0 < jn; k0 += kNbThreads) {
             const int kn = min(32, jn - k0), jb = item.w + j0 + k0;
             const unsigned m = j0 + k0 == 32 * wp ? m0 : group_mask(jb, kn);
             float ax = 0.f, ay = 0.f, az = 0.f;
+            const bool toward = __all_sync(0xffffffffu, lane >= kn || in_box(sm.x[k0 + lane], L));
             // the pair (i, staged partner k0 + k).  MASKED: an excluded pair keeps
             // the IS-SPA correction only, the self pair gets d2 = 1 and adds
             // nothing, both by selects, so that the loop stays unrolled
-            auto pair = [&](int k, auto masked) {
+            auto pair = [&](int k, auto masked, auto side) {
+                constexpr bool T = decltype(side)::value;
                 constexpr bool MASKED = decltype(masked)::value;
                 const bool bit = MASKED && ((m >> k) & 1u);
                 const bool self = MASKED && jb + k == i;
                 const float4 xj = sm.x[k0 + k], c = sm.c[k0 + k];
-                const float rx = mimg(xi.x - xj.x, L, h);
-                const float ry = mimg(xi.y - xj.y, L, h);
-                const float rz = mimg(xi.z - xj.z, L, h);
+                const float rx = image<T>(xi.x - xj.x, sx, L, h);
+                const float ry = image<T>(xi.y - xj.y, sy, L, h);
+                const float rz = image<T>(xi.z - xj.z, sz, L, h);
                 const float d2 = self ? 1.0f : dist2f(rx, ry, rz);
                 const float ri = rsqrtf(d2);
                 const float ri2 = ri * ri;
@@ -146,17 +152,17 @@ __device__ __forceinline__ void nonbond_range(const NonbondArgs &a, int4 item, i
             if (__any_sync(0xffffffffu, m != 0u)) {
                 if (kn == 32) {
 #pragma unroll 4
-                    for (int k = 0; k < 32; ++k) pair(k, std::true_type{});
+                    for (int k = 0; k < 32; ++k) pair(k, std::true_type{}, std::false_type{});
                 } else {
 #pragma unroll 1
-                    for (int k = 0; k < kn; ++k) pair(k, std::true_type{});
+                    for (int k = 0; k < kn; ++k) pair(k, std::true_type{}, std::false_type{});
                 }
-            } else if (kn == 32) {
+            } else if (kn == 32 && toward) {
 #pragma unroll 8
-                for (int k = 0; k < 32; ++k) pair(k, std::false_type{});
+                for (int k = 0; k < 32; ++k) pair(k, std::false_type{}, std::true_type{});
             } else {
 #pragma unroll 1
-                for (int k = 0; k < kn; ++k) pair(k, std::false_type{});
+                for (int k = 0; k < kn; ++k) pair(k, std::false_type{}, std::false_type{});
             }
             if (active) check_force(a.status, ax, ay, az);
             f[0] += to_fix(ax);
