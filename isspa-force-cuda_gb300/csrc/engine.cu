@@ -91,6 +91,8 @@ struct isspa_engine {
     int n_force_items = 0, force_chunk = 0;
     int force_tail = 0;  // chunk length of the short items listed last (0: none)
     int field_vote = 0;  // field pass in warp-voted groups of four atoms
+    bool field_auto = false;      // ... or by size, the option not given and no autotuning
+    float box_over_rmax = 0.0f;   // of the widest window
     int field_tma = 0;   // field pass stages its atom rounds by 1-D bulk copies (TMA)
     int step_pdl = 0;    // step chain launched as programmatic dependents (1) or not (0)
     int isspa_fused = 0;  // field and force passes as one launch (1) when fused_ok()
@@ -209,11 +211,6 @@ struct isspa_engine {
     // Windows in descending size, so the costliest tiles are scheduled first.
     std::vector<int> order;
 
-    static double wave_eff(long long units, long long slots) {
-        if (slots <= 0 || units <= 0) return 0.0;
-        const double waves = (double)units / (double)slots;
-        return waves / std::ceil(waves);
-    }
     long long field_tiles_for(int S) const {
         const int tp = field_points_per_block(S);
         long long n = 0;
@@ -231,18 +228,8 @@ struct isspa_engine {
         return default_split(n_sms, [&](int S) { return field_tiles_for(S); });
     }
     int default_force_chunk() const {
-        const long long slots = (long long)n_sms * std::max(1, force_blocks_per_sm(force_apt));
-        double best = -1.0;
-        int C = 64;
-        for (long long c = 8192; c >= 32; --c) {  // longest chunk (fewest atomics) at equal efficiency
-            const long long n = force_items_for(c);
-            const double e = n < slots ? 0.5 * (double)n / (double)slots : wave_eff(n, slots);
-            if (e > best + 0.005) {
-                best = e;
-                C = (int)c;
-            }
-        }
-        return C;
+        return default_chunk((long long)n_sms * std::max(1, force_blocks_per_sm(force_apt)),
+                             [&](long long C) { return force_items_for(C); });
     }
     void set_field_split(int S) {
         std::vector<int4> t;
@@ -374,7 +361,7 @@ struct isspa_engine {
     // ---------------------------------------------------------------- args
     FieldArgs field_args() const {
         FieldArgs a{};
-        a.vote = field_vote;
+        a.vote = field_vote || (field_auto && default_vote(field_split, box_over_rmax));
         a.tma = field_tma;
         a.pos = pos;
         a.atype = atype;
@@ -1152,6 +1139,11 @@ void build(isspa_engine &E, const std::vector<isspa_host_system> &ws) {
     if (S != 1 && S != 2 && S != 4 && S != 8 && S != 16) S = E.default_field_split();
     E.set_field_split(S);
     E.field_vote = E.opt.field_vote == 1 ? 1 : 0;
+    E.field_auto = E.opt.field_vote == 0;
+    float box = 0.0f, rmax = 0.0f;
+    for (const WinDev &d : E.win_h) box = std::max(box, d.box);
+    for (float x : f0.rmax) rmax = std::max(rmax, x);
+    E.box_over_rmax = rmax > 0.0f ? box / rmax : 0.0f;
     E.field_tma = E.opt.field_tma == 1 ? 1 : 0;
     // (programmatic launches unasked for where the chain is nonbond and update
     // alone: 1100 / 4400 / 8800 atoms 10.8 -> 10.1, 36.2 -> 34.0, 109 -> 106 us)
@@ -1780,6 +1772,7 @@ int isspa_autotune(isspa_engine *e, int reps, int shape[ISSPA_SHAPE_COUNT]) {
             ck(cudaEventElapsedTime(&ms, e->ev_a, e->ev_b));
             return ms / reps;
         };
+        e->field_auto = false;
         // field pass: every atom-loop split, per-pair and warp-voted loops,
         // atom rounds staged by plain loads and by bulk copies (TMA)
         float best = 1e30f;

@@ -189,36 +189,58 @@ extern "C" int isspa_force_noalloc(const isspa_noalloc_inputs *in_p, float *forc
     int rc = scratch_address(&base, &sms);
     if (rc) return rc;
 
-    // launch shapes: the engine's default field split, force chunks for >= 2 waves
-    const int S = default_split(sms, [&](int c) { return (P + field_points_per_block(c) - 1) / field_points_per_block(c); });
-    Plan pl{};
-    pl.n_atoms = in.n_atoms;
-    pl.tp = field_points_per_block(S);
-    pl.P = P;
-    pl.atiles = (in.n_atoms + 127) / 128;
-    const long long fslots = (long long)sms * std::max(1, force_blocks_per_sm(1));
-    pl.C = std::max<long long>(64, std::min<long long>(8192, (pl.atiles * P + 2 * fslots - 1) / (2 * fslots)));
-    pl.n_tiles = (P + pl.tp - 1) / pl.tp;
-    pl.n_chunks = (P + pl.C - 1) / pl.C;
-    pl.n_items = pl.atiles * pl.n_chunks;
-
-    // scratch layout
+    // launch shapes: the engine's defaults where they fit the buffer, else longer
+    // chunks and whole waves of tiles (shorter lists; these decide what fits)
     const int nt = in.n_isspa_types;
-    Layout L;
-    const size_t o_win = L.take(sizeof(WinDev));
-    const size_t o_tiles = L.take(sizeof(int4) * pl.n_tiles);
-    const size_t o_items = L.take(sizeof(int4) * pl.n_items);
-    const size_t o_chunks = L.take(sizeof(int2) * pl.n_chunks);
-    const size_t o_gtab = L.take(sizeof(float4) * (size_t)nt * (in.n_g - 1));
-    const size_t o_ftab = L.take(sizeof(float2) * (size_t)nt * in.n_f);
-    const size_t o_vtot = L.take(sizeof(float) * nt);
-    const size_t o_atype = L.take(sizeof(int2) * in.n_atoms);
-    const size_t o_facc = L.take(sizeof(unsigned long long) * 3 * (size_t)in.n_atoms);
-    size_t o_q[5];
-    for (int k = 0; k < 5; ++k) o_q[k] = L.take(sizeof(float4) * (size_t)P);
-    const size_t o_step = L.take(sizeof(uint32_t));
-    const size_t o_status = L.take(sizeof(int));
-    if (L.off > ISSPA_NOALLOC_SCRATCH_BYTES) return ISSPA_ERR_UNSUPPORTED;
+    Plan pl{};
+    size_t o_win, o_tiles, o_items, o_chunks, o_gtab, o_ftab, o_vtot, o_atype, o_facc, o_q[5], o_step, o_status;
+    auto tiles = [&](int S) { return (P + field_points_per_block(S) - 1) / field_points_per_block(S); };
+    auto lay_out = [&](int S, long long C) {  // the plan and its scratch bytes
+        pl.n_atoms = in.n_atoms;
+        pl.tp = field_points_per_block(S);
+        pl.P = P;
+        pl.atiles = (in.n_atoms + 127) / 128;
+        pl.C = C;
+        pl.n_tiles = tiles(S);
+        pl.n_chunks = (P + C - 1) / C;
+        pl.n_items = pl.atiles * pl.n_chunks;
+        Layout L;
+        o_win = L.take(sizeof(WinDev));
+        o_tiles = L.take(sizeof(int4) * pl.n_tiles);
+        o_items = L.take(sizeof(int4) * pl.n_items);
+        o_chunks = L.take(sizeof(int2) * pl.n_chunks);
+        o_gtab = L.take(sizeof(float4) * (size_t)nt * (in.n_g - 1));
+        o_ftab = L.take(sizeof(float2) * (size_t)nt * in.n_f);
+        o_vtot = L.take(sizeof(float) * nt);
+        o_atype = L.take(sizeof(int2) * in.n_atoms);
+        o_facc = L.take(sizeof(unsigned long long) * 3 * (size_t)in.n_atoms);
+        for (int k = 0; k < 5; ++k) o_q[k] = L.take(sizeof(float4) * (size_t)P);
+        o_step = L.take(sizeof(uint32_t));
+        o_status = L.take(sizeof(int));
+        return L.off;
+    };
+    const long long atiles = (in.n_atoms + 127) / 128;
+    int S = 4;
+    double best = -1.0;
+    for (int c : {1, 2, 4, 8, 16}) {
+        const double waves = (double)tiles(c) / (double)((long long)sms * std::max(1, field_blocks_per_sm(c)));
+        if (waves / std::ceil(waves) > best + 0.02) {
+            best = waves / std::ceil(waves);
+            S = c;
+        }
+    }
+    const long long two_waves = 20LL * sms;
+    if (lay_out(S, std::max<long long>(64, std::min<long long>(8192, (atiles * P + two_waves - 1) / two_waves))) >
+        ISSPA_NOALLOC_SCRATCH_BYTES)
+        return ISSPA_ERR_UNSUPPORTED;
+    const Plan compact = pl;
+    const int S_compact = S;
+    S = default_split(sms, tiles);
+    if (lay_out(S, default_chunk((long long)sms * std::max(1, force_blocks_per_sm(1)),
+                                 [&](long long C) { return atiles * ((P + C - 1) / C); })) > ISSPA_NOALLOC_SCRATCH_BYTES) {
+        S = S_compact;
+        lay_out(S, compact.C);
+    }
     unsigned char *b = static_cast<unsigned char *>(base);
     int *status = (int *)(b + o_status);
 
@@ -271,6 +293,7 @@ extern "C" int isspa_force_noalloc(const isspa_noalloc_inputs *in_p, float *forc
     fa.out = pts;
     fa.terms = terms;
     fa.status = status;
+    fa.vote = default_vote(S, 0.0f);  // (rmax is on the device)
     launch_field(fa, S, false, stream);
 
     ForceArgs ka{};

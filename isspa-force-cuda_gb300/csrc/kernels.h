@@ -383,11 +383,12 @@ int nonbond_block_threads();
 int field_points_per_block(int split);
 int field_blocks_per_sm(int split);
 // The field pass's default split.  A pair costs less the fewer warps share a
-// tile (8800 atoms, S = 1 / 2 / 4 / 8 / 16: 6.02 / 6.59 / 6.95 / 6.76 / 6.99 ms;
-// 1100 atoms 123 / 101 / 96 / 89 / 95 us; 264 atoms 54 / 33 / 24 / 17 / 16.5), as
-// long as the tiles fill the chip: whole waves of resident blocks count, and
-// whole rounds of SMs, since a last wave's blocks run faster for being few.
-// tiles(S): a split's number of tiles.
+// tile, as long as the tiles fill the chip: whole waves of resident blocks count,
+// and whole rounds of SMs, since a last wave's blocks run faster for being few.
+// Us per launch at S = 1 / 2 / 4 / 8 / 16: 8800 atoms (nMC 100) 5496 / 5867 / 6223 /
+// 6402 / 6850, 4400 930 / 832 / 870 / 890 / 962, windows of 44 to 1100 atoms 292 /
+// 299 / 312 / 326 / 387, 1100 atoms 107 / 91 / 88 / 87 / 95, 741 79 / 52 / 42 / 43 /
+// 43, 264 54 / 33 / 24 / 17 / 16.5.  tiles(S): a split's number of tiles.
 template <class Tiles>
 int default_split(int sms, const Tiles &tiles) {
     auto whole = [](long long units, long long slots) {  // filled share of the rounds
@@ -395,7 +396,7 @@ int default_split(int sms, const Tiles &tiles) {
         return (double)units / (double)((units + slots - 1) / slots * slots);
     };
     constexpr int kSplit[5] = {1, 2, 4, 8, 16};
-    constexpr double kCost[5] = {1.0, 1.07, 1.1, 1.1, 1.22};
+    constexpr double kCost[5] = {1.0, 1.13, 1.12, 1.16, 1.35};
     int S = 4;
     double best = -1.0;
     for (int k = 0; k < 5; ++k) {
@@ -407,6 +408,23 @@ int default_split(int sms, const Tiles &tiles) {
         }
     }
     return S;
+}
+// Whether the field pass takes its atoms in voted groups unless told: with few
+// warps a tile always (1100 atoms at S = 4 92.6 -> 87.8 us), with many where the
+// box is wide enough for most groups to lie outside rmax (S = 8: 1100 atoms, box
+// 5 rmax, 87.3 either way, S = 16 94.5 -> 97.3; 4400 atoms, 7.9 rmax, 938 -> 890).
+inline bool default_vote(int split, float box_over_rmax) { return split <= 4 || box_over_rmax >= 6.5f; }
+// The force pass's default chunk: short items balance and overlap their staging,
+// down to a stage's half; below that an item's start counts, unless they are
+// needed to fill the chip.  Us per launch at C = 32 / 48 / 64 / 128 / 256 / 1024: 8800
+// atoms 12 294 / 11 953 / 11 738 / 11 467 / 11 439 / 11 529, 4400 1601 / 1560 / 1533 /
+// 1504 / 1514 / 1600, 1100 124 / 123 / 123 / 129 / 147 / 220, 741 63 / 53 / 54 / 64 /
+// 75 / 174, 264 16 / 18 / 20 / 31 / 49 / 162.  items(C): a chunk's number of items.
+template <class Items>
+int default_chunk(long long slots, const Items &items) {
+    for (int C : {256, 128, 64})
+        if (items(C) >= 6 * slots) return C;
+    return items(48) >= 2 * slots ? 48 : 32;
 }
 int force_blocks_per_sm(int atoms_per_thread);
 int nonbond_blocks_per_sm(int n_lj_types);
