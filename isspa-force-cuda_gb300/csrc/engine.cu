@@ -790,11 +790,13 @@ struct isspa_engine {
         }
         if (bonded_branch) {
             mark(ISSPA_K_BONDED, 0, side);
+            PdlScope branch(false);
             launch_bonded(bonded_args(1, 1, 1), side);
             mark(ISSPA_K_BONDED, 1, side);
         }
         if (us_branch) {
             mark(ISSPA_K_UMBRELLA, 0, side3);
+            PdlScope branch(false);
             launch_umbrella(umbrella_args(), side3);
             mark(ISSPA_K_UMBRELLA, 1, side3);
             ck(cudaEventRecord(ev_join3, side3));
@@ -1334,13 +1336,16 @@ int run_guarded(F &&f) {
     }
 }
 
-// Times `f` with CUDA events on the engine stream when ms_out is given.
+// Times `f` with CUDA events on the engine stream when ms_out is given; else its
+// kernels are programmatic dependents of the calls' before it (a force call of 264
+// atoms, six kernels in a row, takes 59.5 us, 66.1 with a boundary between each).
 template <typename F>
 int timed_call(isspa_engine *e, float *ms_out, F &&f) {
     int rc = guard(e);
     if (rc) return rc;
     return run_guarded([&] {
         if (ms_out) ck(cudaEventRecord(e->ev_a, e->stream));
+        PdlScope pdl(!ms_out);
         f();
         ck(cudaGetLastError());
         if (ms_out) {

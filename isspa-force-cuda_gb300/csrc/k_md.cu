@@ -43,6 +43,8 @@ __global__ void __launch_bounds__(kNbThreads, 8) nonbond_kernel(NonbondArgs a, B
 }
 
 __global__ void bonded_kernel(BondedArgs a) {
+    pdl_wait();
+    pdl_trigger();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     bonded_term(a, idx, FixAdd{a.facc, a.status});
 }
@@ -50,7 +52,10 @@ __global__ void bonded_kernel(BondedArgs a) {
 __global__ void __launch_bounds__(kUsThreads) umbrella_kernel(UmbrellaArgs a) {
     __shared__ double s_red[6 * kUsThreads];
     __shared__ double s_f[4];
-    umbrella_window(a, a.us_windows[blockIdx.x], s_red, s_f, [] {});
+    umbrella_window(a, a.us_windows[blockIdx.x], s_red, s_f, [] {
+        pdl_wait();
+        pdl_trigger();
+    });
 }
 
 // Every block reads the step counter first; the last block to finish
@@ -198,11 +203,11 @@ int nonbond_blocks_per_sm(int n_lj_types) {
 
 void launch_bonded(const BondedArgs &a, cudaStream_t s) {
     const int tpb = 128, blocks = bonded_blocks(a, tpb);
-    if (blocks > 0) bonded_kernel<<<blocks, tpb, 0, s>>>(a);
+    if (blocks > 0) launch_chain(bonded_kernel, blocks, tpb, s, a);
 }
 
 void launch_umbrella(const UmbrellaArgs &a, cudaStream_t s) {
-    if (a.n_us_windows > 0) umbrella_kernel<<<a.n_us_windows, kUsThreads, 0, s>>>(a);
+    if (a.n_us_windows > 0) launch_chain(umbrella_kernel, a.n_us_windows, kUsThreads, s, a);
 }
 
 int integrator_block_threads() { return kUsThreads; }
