@@ -739,8 +739,11 @@ struct isspa_engine {
             if (timed && launches(k)) ck(cudaEventRecordWithFlags(kev[2 * k + end], s, cudaEventRecordExternal));
         };
         // programmatic launches for the field -> force -> leapfrog chain (not
-        // in the event-instrumented copy, whose event nodes sit between them)
-        PdlScope pdl(step_pdl == 1 && !timed && integrator != 3);
+        // in the event-instrumented copy, whose event nodes sit between them);
+        // merged steps unasked: autotuning times graphs of one step, where they
+        // do not show (back to back 44 / ADI2 / 264 atoms 7.4 / 9.5 / 20.8 us, 8.9 /
+        // 10.6 / 22.5 without)
+        PdlScope pdl((step_pdl == 1 || (opt.step_pdl == 0 && merged())) && !timed && integrator != 3);
         if (integrator == 3) {  // the whole step in one cooperative kernel
             mark(ISSPA_K_STEP, 0, stream);
             if (n_atoms > 0) ck(launch_step(step_args(), step_grid(), stream));
