@@ -159,7 +159,8 @@ typedef struct isspa_engine_options {
                               (each waits for that kernel's completion before its first memory
                               access, so its launch overlaps the other's tail; same results);
                               2: ordinary launches; 0 => 2 until isspa_autotune times both and
-                              keeps the faster.  The single-kernel step has no chain */
+                              keeps the faster, but 1 for steps of one merged launch and for
+                              engines without IS-SPA terms.  The single-kernel step has no chain */
     int isspa_fused;       /* 1: the field and force passes run as one launch over the field
                               tiles: each block computes its points' fields, then those points'
                               forces on every atom of its window (for small windows; needs

@@ -407,10 +407,10 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, F
         // any of them inside rmax.  When none does, their out-of-range Coulomb
         // terms are summed without per-pair branches; the accumulators see the
         // same operations in the same order either way.  It pays where few
-        // groups have an atom in range (large systems: 16 384 atoms in a
-        // 120 A box, 21.5 against 23.4 ms per launch) and costs registers
-        // where many do (1100 atoms: 0.092 against 0.087 ms), so the
-        // autotuner chooses.
+        // groups have an atom in range and where few warps share a tile (8800
+        // atoms, S = 1, 5496 against 6083 us per launch; 1100 atoms, S = 4, 87.8
+        // against 92.6), and costs registers where neither holds (1100 atoms,
+        // S = 16, 97.3 against 94.5): default_vote, or the autotuner's choice.
         constexpr int kG = 4;
         for (; VOTE && k + (kG - 1) * S < jn; k += kG * S) {
             float rx[kG], ry[kG], rz[kG], c[kG];
