@@ -945,7 +945,8 @@ __global__ void __launch_bounds__(FieldShape<S>::kThreads, 1024 / FieldShape<S>:
 // Per back-to-back step, the branched graph of the fused launch before and this
 // (best field split): 44 atoms nMC 20 10.6 -> 8.0 us, ADI2 (44 atoms, nMC 100,
 // restrained) 11.3 -> 9.9, 132 atoms 15.8 -> 11.5, 264 atoms 23.7 -> 22.5, four
-// windows of 44 atoms 11.8 -> 8.5.  What is left of a 44-atom step, from
+// windows of 44 atoms 11.8 -> 8.5 (with the pair loops and the update as they are
+// now 7.4, 9.5 and, 264 atoms, 20.8).  What is left of a 44-atom step, from
 // %globaltimer: 0.9 us positions and draws, 0.9 atom loop, 0.7 sums and
 // Langevin, 1.4 forces, 0.8 to the integrator's sight (fence, count, poll), 1.3
 // its read of the sums and update, 1.3 to the next step's start -- L2 round

@@ -27,11 +27,12 @@ constexpr int kNbMaxAB = 4096;  // LJ type pairs held in shared memory (up to 64
 // runs without per-pair checks.
 //
 // A lane used to take all 128 partners of a stage, and a small system waits for
-// that chain.  Four warps on one row tile cut it to 32 pairs: a solvent-free step
+// that chain.  Four warps on one row tile cut it to 32 pairs: a solvent-free step,
+// the pass on a branch of it,
 // of 264 / 1100 / 2200 / 3300 atoms takes 9.5 / 10.0 / 15.9 / 23.8 us, with a
 // thread per row 12.4 / 13.1 / 18.7 / 35.3.  From about 4400 atoms on the pass is
-// bound by issue (83 % of the slots, 43 instructions per 32 pairs, most of them
-// the image's compare and select and the pair's multiplies), and the pair counts:
+// bound by issue (83 % of the slots, 43 instructions per 32 pairs, 40 since the
+// image's direction is settled by the row), and the pair counts:
 // every term shares q_i q_j, the staged constants fold the correction into two
 // multiply-adds and the LJ table holds 12 A and -6 B (4400 / 8800 atoms: 34.8 /
 // 107.6 us, before 36.7 / 111.4).
