@@ -27,14 +27,13 @@ constexpr int kNbMaxAB = 4096;  // LJ type pairs held in shared memory (up to 64
 // runs without per-pair checks.
 //
 // A lane used to take all 128 partners of a stage, and a small system waits for
-// that chain.  Four warps on one row tile cut it to 32 pairs: a solvent-free step,
-// the pass on a branch of it,
-// of 264 / 1100 / 2200 / 3300 atoms takes 9.5 / 10.0 / 15.9 / 23.8 us, with a
-// thread per row 12.4 / 13.1 / 18.7 / 35.3.  From about 4400 atoms on the pass is
-// bound by issue (83 % of the slots, 43 instructions per 32 pairs, 40 since the
-// image's direction is settled by the row), and the pair counts:
-// every term shares q_i q_j, the staged constants fold the correction into two
-// multiply-adds and the LJ table holds 12 A and -6 B (4400 / 8800 atoms: 34.8 /
+// that chain.  Four warps on one row tile cut it to 32 pairs: a solvent-free step
+// of 264 / 1100 / 2200 / 3300 atoms, the pass on a branch of it, takes 9.5 / 10.0 /
+// 15.9 / 23.8 us, with a thread per row 12.4 / 13.1 / 18.7 / 35.3.  From about 4400
+// atoms on the pass is bound by issue (83 % of the slots, 43 instructions per 32
+// pairs, 40 since the image's direction is settled by the row), and the pair
+// counts: every term shares q_i q_j, the staged constants fold the correction into
+// two multiply-adds and the LJ table holds 12 A and -6 B (4400 / 8800 atoms: 34.8 /
 // 107.6 us, before 36.7 / 111.4).
 // SMEM_AB: that table of every ordered type pair sits in shared memory
 // (dynamic, nt^2 float2) instead of a global gather per pair.  ALL: every term
