@@ -313,10 +313,12 @@ int isspa_device_status(isspa_engine *e, int reset);
  * Synchronises the engine stream.  ISSPA_ERR_STATE without a cutoff. */
 int isspa_nonbond_list_stats(isspa_engine *e, int *builds, int *fullest_row);
 /* Failure-detection testing (no counterpart in the reference): leaves the
- * fused integrator's grid barrier as if a block had been lost mid-count, so the
- * next fused step's bounded waits run out; that step integrates nothing and
- * reports ISSPA_ERR_TIMEOUT through isspa_device_status, whose reset also
- * restores the barrier.  No kernel faults and the context stays usable. */
+ * fused integrator's grid barrier, and the completion count of an engine that
+ * steps by one merged launch, as if a block had been lost mid-count, so the
+ * next such step's bounded waits run out; that step and those queued behind it
+ * integrate nothing and report ISSPA_ERR_TIMEOUT through isspa_device_status,
+ * whose reset also restores the barrier or count and clears the force
+ * accumulator.  No kernel faults and the context stays usable. */
 int isspa_debug_stall_barrier(isspa_engine *e);
 
 /* ---- state transfer (host <-> device, synchronous) ----------------------- */

@@ -2129,10 +2129,12 @@ int isspa_device_status(isspa_engine *e, int reset) {
         cudaGetLastError();
         return ISSPA_ERR_CUDA;
     }
-    // a grid barrier or a merged step that gave up leaves its count: reset with the status
+    // a grid barrier or a merged step that gave up leaves its count and the
+    // forces of the steps that did not integrate: reset with the status
     if (reset && (cudaMemsetAsync(e->status, 0, sizeof(int), e->stream) != cudaSuccess ||
                   ((st & kStatusTimeout) && (cudaMemsetAsync(e->bar, 0, 2 * sizeof(unsigned int), e->stream) != cudaSuccess ||
                                              cudaMemsetAsync(e->d_done, 0, sizeof(unsigned int), e->stream) != cudaSuccess ||
+                                             cudaMemsetAsync(e->facc, 0, 3 * sizeof(unsigned long long) * e->n_atoms, e->stream) != cudaSuccess ||
                                              (e->mg_copies && cudaMemsetAsync(e->mg_copies, 0, sizeof(unsigned long long) * e->mg_copy_words(), e->stream) != cudaSuccess))) ||
                   cudaStreamSynchronize(e->stream) != cudaSuccess)) {
         cudaGetLastError();
@@ -2170,6 +2172,8 @@ int isspa_debug_stall_barrier(isspa_engine *e) {
         // an arrival count no grid reaches: every block waits out its limit
         const unsigned int words[2] = {0x80000000u, 0u};
         ck(cudaMemcpyAsync(e->bar, words, sizeof words, cudaMemcpyHostToDevice, e->stream));
+        // (only the merged step waits for the completion count)
+        if (e->merged()) ck(cudaMemcpyAsync(e->d_done, words, sizeof(unsigned int), cudaMemcpyHostToDevice, e->stream));
         ck(cudaStreamSynchronize(e->stream));
     });
 }

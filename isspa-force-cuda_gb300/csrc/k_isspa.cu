@@ -984,17 +984,19 @@ __global__ void __launch_bounds__(FieldShape<S>::kThreads, 1024 / FieldShape<S>:
         LeapfrogAtom first = {};
         if (threadIdx.x < m.lf.n_atoms) first = leapfrog_prepare(m.lf, threadIdx.x, step);
         if (threadIdx.x == 0) {
-            s_ok = 1;
+            // a step that gave up leaves the count and the accumulators
+            // mid-step: no step behind it integrates before the status reset,
+            // which clears them
+            s_ok = !(__ldcg(m.lf.status) & kStatusTimeout);
             const unsigned long long t0 = global_ns();
-            while (ld_acquire_u32(m.lf.done_ptr) != gridDim.x - 1)
+            while (s_ok && ld_acquire_u32(m.lf.done_ptr) != gridDim.x - 1)
                 if (global_ns() - t0 > kBarrierWaitNs) {
                     atomicOr(m.lf.status, kStatusTimeout);
                     s_ok = 0;
-                    break;
                 }
         }
         __syncthreads();
-        if (!s_ok) return;  // (the status reset clears the count)
+        if (!s_ok) return;
         for (int i = threadIdx.x; i < m.lf.n_atoms; i += kT) {
             // the other copies of the accumulator: read all at once, cleared
             long long extra[3] = {0, 0, 0}, c[kMergedCopies - 1][3];
