@@ -971,7 +971,9 @@ struct MergedSmem {
 template <int S, bool NB_ALL, bool TS>
 __global__ void __launch_bounds__(FieldShape<S>::kThreads, 1024 / FieldShape<S>::kThreads) merged_step_kernel(MergedArgs m) {
     constexpr int kT = FieldShape<S>::kThreads;
-    extern __shared__ unsigned char s_dyn[];
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    static_assert(alignof(MergedSmem<S>) <= 16 && sizeof(MergedSmem<S>) % 16 == 0,
+                  "the float4 tables follow the buffers at 16 bytes");
     MergedSmem<S> &sm = *reinterpret_cast<MergedSmem<S> *>(s_dyn);
     int b = blockIdx.x;
     if (b == 0) {
