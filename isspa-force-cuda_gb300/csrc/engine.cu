@@ -580,7 +580,7 @@ struct isspa_engine {
     // (or no IS-SPA pass); other engines step with separate kernels.
     bool step_kernel_ok() const {
         return n_atoms > 0 && !inject && !cutoff && n_lj_types * n_lj_types <= 4096 &&
-               (opt.isspa_terms == 0 || (opt.isspa_terms & 2)) && force_apt == 1;
+               (opt.isspa_terms == 0 || (opt.isspa_terms & 2)) && force_apt == 1 && step_max_blocks(n_lj_types) > 0;
     }
     StepArgs step_args() const {
         StepArgs a{};

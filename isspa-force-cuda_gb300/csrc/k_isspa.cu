@@ -1175,7 +1175,12 @@ int step_threads() { return kFieldThreads; }
 int step_max_blocks(int n_lj_types) {
     int dev = 0, sms = 0, per_a = 0, per_b = 0;
     const size_t smem = sizeof(float2) * (size_t)std::max(1, n_lj_types * n_lj_types);
+    // the table beside the phases' buffers (39 KB): from 34 types on more than
+    // the default 48 KB a block
+    const cudaFuncAttribute limit = cudaFuncAttributeMaxDynamicSharedMemorySize;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(step_kernel<true>, limit, (int)(sizeof(float2) * kNbMaxAB)) != cudaSuccess ||
+        cudaFuncSetAttribute(step_kernel<false>, limit, (int)(sizeof(float2) * kNbMaxAB)) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_a, step_kernel<true>, kFieldThreads, smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_b, step_kernel<false>, kFieldThreads, smem) != cudaSuccess) {
         cudaGetLastError();
