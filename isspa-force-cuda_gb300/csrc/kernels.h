@@ -420,10 +420,19 @@ inline bool default_vote(int split, float box_over_rmax) { return split <= 4 || 
 // atoms 12 294 / 11 953 / 11 738 / 11 467 / 11 439 / 11 529, 4400 1601 / 1560 / 1533 /
 // 1504 / 1514 / 1600, 1100 124 / 123 / 123 / 129 / 147 / 220, 741 63 / 53 / 54 / 64 /
 // 75 / 174, 264 16 / 18 / 20 / 31 / 49 / 162.  items(C): a chunk's number of items.
+// The list grows with atoms x points: past kMaxListedItems (16 MB) the chunks
+// lengthen instead (1 M atoms, nMC 100: 3e9 items of 256 points would not fit the
+// item count).
+constexpr long long kMaxListedItems = 1ll << 20;
+template <class Items>
+int bounded_chunk(int C, const Items &items) {
+    while (C < 1 << 30 && items(C) > kMaxListedItems) C *= 2;
+    return C;
+}
 template <class Items>
 int default_chunk(long long slots, const Items &items) {
     for (int C : {256, 128, 64})
-        if (items(C) >= 6 * slots) return C;
+        if (items(C) >= 6 * slots) return bounded_chunk(C, items);
     return items(48) >= 2 * slots ? 48 : 32;
 }
 int force_blocks_per_sm(int atoms_per_thread);
