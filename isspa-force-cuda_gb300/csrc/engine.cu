@@ -1553,24 +1553,34 @@ int isspa_adjoint_mean_force(isspa_engine *e, int n_frames, const float *frames,
         }
         // J weighs restrained atoms only: the IS-SPA force pass runs on the 128-atom
         // tiles that hold one (16 windows x 550 atoms: one tile of five), in
-        // chunks of 128 points so that those tiles alone fill the GPU
+        // chunks of 128 points so that those tiles alone fill the GPU (a multiple
+        // of 128 for the largest systems: bounded_chunk)
         if (!e->adj_items) {
             std::vector<char> biased(N, 0);
             for (const int2 &b : e->bias_h) biased[b.x] = 1;
+            std::vector<std::vector<int>> tiles(W);  // first atom within the window
+            for (int w = 0; w < W; ++w) {
+                const WinDev &d = e->win_h[w];
+                for (int t = 0; t < d.n_atoms; t += 128) {
+                    const auto first = biased.begin() + d.atom_off + t, last = first + std::min(128, d.n_atoms - t);
+                    if (std::find(first, last, 1) != last) tiles[w].push_back(t);
+                }
+            }
+            const int len = bounded_chunk(128, [&](long long C) {
+                long long n = 0;
+                for (int w = 0; w < W; ++w)
+                    n += (long long)tiles[w].size() * (((long long)e->win_h[w].n_atoms * e->n_mc + C - 1) / C);
+                return n;
+            });
             std::vector<int4> items;
             std::vector<int2> chunks;
             for (int w = 0; w < W; ++w) {
                 const WinDev &d = e->win_h[w];
-                std::vector<int> tiles;
-                for (int t = 0; t < d.n_atoms; t += 128) {
-                    const auto first = biased.begin() + d.atom_off + t, last = first + std::min(128, d.n_atoms - t);
-                    if (std::find(first, last, 1) != last) tiles.push_back(t);
-                }
                 const long long np = (long long)d.n_atoms * e->n_mc;
-                for (long long p = 0; !tiles.empty() && p < np; p += 128) {
-                    for (int t : tiles)
+                for (long long p = 0; !tiles[w].empty() && p < np; p += len) {
+                    for (int t : tiles[w])
                         items.push_back(make_int4(w, d.atom_off + t, std::min(128, d.n_atoms - t), (int)chunks.size()));
-                    chunks.push_back(make_int2((int)(d.point_off + p), (int)std::min<long long>(128, np - p)));
+                    chunks.push_back(make_int2((int)(d.point_off + p), (int)std::min<long long>(len, np - p)));
                 }
             }
             e->adj_chunks = e->upload(chunks);
