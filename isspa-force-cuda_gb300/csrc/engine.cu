@@ -148,7 +148,8 @@ struct isspa_engine {
     // adjoint buffers (allocated on first use)
     int4 *adj_items = nullptr;  // force work items of the tiles that hold a restrained atom
     int2 *adj_chunks = nullptr;
-    int n_adj_items = 0;
+    int2 *adj_tiles = nullptr;  // point tiles of the restrained windows
+    int n_adj_items = 0, n_adj_tiles = 0;
     int *adj_off = nullptr, *adj_atoms = nullptr;
     double *adj_s = nullptr, *axis = nullptr;
     double *cvec = nullptr, *lam = nullptr, *grads = nullptr;
@@ -1551,6 +1552,15 @@ int isspa_adjoint_mean_force(isspa_engine *e, int n_frames, const float *frames,
             e->adj_s = e->alloc<double>(std::max<size_t>(1, e->bias_h.size()));
             e->axis = e->alloc<double>(3 * (size_t)W);
         }
+        if (!e->adj_tiles) {
+            std::vector<int2> tiles;
+            for (int w = 0; w < W; ++w)
+                for (long long p = 0; e->win_h[w].us_on && p < (long long)e->win_h[w].n_atoms * e->n_mc;
+                     p += adjoint_point_tile())
+                    tiles.push_back(make_int2(w, (int)p));
+            e->adj_tiles = e->upload(tiles);
+            e->n_adj_tiles = (int)tiles.size();
+        }
         // J weighs restrained atoms only: the IS-SPA force pass runs on the 128-atom
         // tiles that hold one (16 windows x 550 atoms: one tile of five), in
         // chunks of 128 points so that those tiles alone fill the GPU (a multiple
@@ -1673,9 +1683,9 @@ int isspa_adjoint_mean_force(isspa_engine *e, int n_frames, const float *frames,
             a.atype = e->atype;
             a.win = e->win;
             a.atom_win = e->atom_win;
-            a.n_windows = W;
+            a.tiles = e->adj_tiles;
+            a.n_tiles = e->n_adj_tiles;
             a.stage = adjoint_stage(e->max_window_atoms());
-            a.tiles_max = (int)(((long long)e->max_window_atoms() * e->n_mc + adjoint_point_tile() - 1) / adjoint_point_tile());
             a.raw_e = e->raw_e;
             a.raw_e0 = e->raw_e0;
             a.q0 = e->pts.q0;

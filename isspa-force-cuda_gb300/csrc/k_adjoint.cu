@@ -80,17 +80,14 @@ __device__ __forceinline__ double widen(float v) {
 }
 __device__ __forceinline__ double df_sum(DF a) { return widen(a.hi) + widen(a.lo); }
 
-// A block's window and point tile: blocks are window-major, tiles_max per
-// window; false when the window has no restraint or no such tile.
-__device__ __forceinline__ bool adj_tile(const AdjointArgs &a, int &w, long long &p, bool &valid) {
-    w = blockIdx.x / a.tiles_max;
-    const long long q = (long long)(blockIdx.x % a.tiles_max) * kAdjThreads;
-    const WinDev &W = a.win[w];
-    const long long n = (long long)W.n_atoms * a.n_mc;
-    if (!W.us_on || q >= n) return false;
-    valid = q + threadIdx.x < n;
-    p = W.point_off + q + (valid ? threadIdx.x : 0);
-    return true;
+// A block's window and point; a lane past the window's points repeats the tile's
+// first (valid false).
+__device__ __forceinline__ void adj_tile(const AdjointArgs &a, int &w, long long &p, bool &valid) {
+    const int2 tile = a.tiles[blockIdx.x];
+    w = tile.x;
+    const WinDev W = a.win[w];
+    valid = (long long)tile.y + threadIdx.x < (long long)W.n_atoms * a.n_mc;
+    p = W.point_off + tile.y + (valid ? threadIdx.x : 0);
 }
 
 // One weighted atom, staged for a block of points: weights c_i = s_i n with n
@@ -113,7 +110,7 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_points_kernel(AdjointArgs
     int w;
     long long p;
     bool valid;
-    if (!adj_tile(a, w, p, valid)) return;
+    adj_tile(a, w, p, valid);
     const WinDev W = a.win[w];
     const float4 raw = a.raw_e[p], raw0 = a.raw_e0[p];
     const float4 P = a.q0[p];
@@ -196,7 +193,7 @@ __global__ void __launch_bounds__(kAdjThreads, 10) adjoint_density_kernel(Adjoin
     int w;
     long long p;
     bool valid;
-    if (!adj_tile(a, w, p, valid)) return;
+    adj_tile(a, w, p, valid);
     const WinDev W = a.win[w];
     const double lam = a.lam[p];
     const float4 P = a.q0[p];
@@ -337,8 +334,8 @@ __global__ void adjoint_14_kernel(AdjointArgs a) {
 }  // namespace
 
 void launch_adjoint(const AdjointArgs &a, cudaStream_t s) {
-    if (a.tiles_max > 0) {
-        const unsigned blocks = (unsigned)((long long)a.tiles_max * a.n_windows);
+    if (a.n_tiles > 0) {
+        const unsigned blocks = (unsigned)a.n_tiles;
         adjoint_points_kernel<<<blocks, kAdjThreads, 0, s>>>(a);
         const size_t smem = (size_t)a.stage * sizeof(float4) + (size_t)(a.stage / 32) * kAdjThreads * sizeof(unsigned);
         adjoint_density_kernel<<<blocks, kAdjThreads, smem, s>>>(a);

@@ -223,7 +223,8 @@ struct AdjointArgs {
     const int2 *atype;
     const WinDev *win;
     const int *atom_win;
-    int n_windows, tiles_max;  // point tiles of the largest window (adjoint_point_tile() points each)
+    const int2 *tiles;         // restrained windows' point tiles: window, first point within it
+    int n_tiles;               // (adjoint_point_tile() points each)
     int stage;                 // atoms the density kernel stages at a time (adjoint_stage)
     const float4 *raw_e;       // field pass: E, w
     const float4 *raw_e0;      // field pass: E0, n

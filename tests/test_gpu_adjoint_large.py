@@ -42,3 +42,23 @@ def test_force_list_is_bounded():
     terms = sign * (f[s.bias_list[:, 0]] @ n)
     assert eng.device_status() == 0
     assert abs(J - terms.sum()) <= 1e-5 * np.abs(terms).sum()
+
+
+def test_windows_of_very_different_sizes():
+    """One restrained window beside a thousand of two atoms, half of them without a
+    restraint: the large one gives what it gives alone, and only the restrained ones
+    have a gradient."""
+    n_mc = 20
+    ff = ig.synth.forcefield(n_mc=n_mc)
+    big = ig.synth.make_system(60, 22, 66.0, n_mc, seed=5, ff=ff, us=(10.0, 5.0))
+    small = [ig.synth.make_system(2, 1, 30.0, n_mc, seed=6 + k, ff=ff, us=(10.0, 6.0) if k else None) for k in range(2)]
+    wins = [big] + [small[k % 2] for k in range(1000)]
+    eng = ig.Engine(wins, field_split=4)  # (the FP32 fields' order is the split's)
+    got = eng.adjoint_mean_force([7])
+    assert eng.device_status() == 0
+    one = ig.Engine(big, field_split=4).adjoint_mean_force([7])
+    for g, r in zip(got, one):  # FP64 sums in another order
+        assert np.allclose(g[0], r[0], rtol=1e-12, atol=1e-12 * np.abs(r[0]).max())
+    for w in (1, 2, 999, 1000):
+        assert (got[0][w] != 0.0) == bool(wins[w].us_on)
+        assert np.any(got[2][w]) == bool(wins[w].us_on)
