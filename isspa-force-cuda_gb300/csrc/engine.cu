@@ -189,6 +189,12 @@ struct isspa_engine {
         allocated += bytes;
         return static_cast<T *>(p);
     }
+    // A buffer kept from its first use on; each has its own check, so that a call
+    // refused part way (over the memory cap) finds the missing ones the next time.
+    template <typename T>
+    void alloc_once(T *&p, size_t n) {
+        if (!p) p = alloc<T>(n);
+    }
     template <typename T>
     T *upload(const std::vector<T> &v) {
         T *p = alloc<T>(v.size());
@@ -652,6 +658,7 @@ struct isspa_engine {
         std::vector<int4> items;
         std::vector<int> nj;
         nonbond_items(merged_nonbond_partners(field_split), items, nj);
+        mg_split = 0;
         release(mg_items);
         release(mg_nj);
         release(mg_copies);
@@ -1539,19 +1546,15 @@ int isspa_adjoint_mean_force(isspa_engine *e, int n_frames, const float *frames,
     std::vector<float4> saved(N);
     uint32_t saved_step = 0;
     rc = run_guarded([&] {
-        if (!e->raw_e) {
-            e->raw_e = e->alloc<float4>(P);
-            e->raw_e0 = e->alloc<float4>(P);
-        }
-        if (!e->cvec) {
-            e->cvec = e->alloc<double>(3 * (size_t)N);
-            e->lam = e->alloc<double>(P);
-            e->grads = e->alloc<double>((size_t)W * per_w);
-            e->adj_off = e->alloc<int>(W + 1);
-            e->adj_atoms = e->alloc<int>(std::max<size_t>(1, e->bias_h.size()));
-            e->adj_s = e->alloc<double>(std::max<size_t>(1, e->bias_h.size()));
-            e->axis = e->alloc<double>(3 * (size_t)W);
-        }
+        e->alloc_once(e->raw_e, P);
+        e->alloc_once(e->raw_e0, P);
+        e->alloc_once(e->cvec, 3 * (size_t)N);
+        e->alloc_once(e->lam, P);
+        e->alloc_once(e->grads, (size_t)W * per_w);
+        e->alloc_once(e->adj_off, W + 1);
+        e->alloc_once(e->adj_atoms, e->bias_h.size());
+        e->alloc_once(e->adj_s, e->bias_h.size());
+        e->alloc_once(e->axis, 3 * (size_t)W);
         if (!e->adj_tiles) {
             std::vector<int2> tiles;
             for (int w = 0; w < W; ++w)
@@ -1593,6 +1596,7 @@ int isspa_adjoint_mean_force(isspa_engine *e, int n_frames, const float *frames,
                     chunks.push_back(make_int2((int)(d.point_off + p), (int)std::min<long long>(len, np - p)));
                 }
             }
+            e->release(e->adj_chunks);  // (of a call refused between the two)
             e->adj_chunks = e->upload(chunks);
             e->adj_items = e->upload(items);
             e->n_adj_items = (int)items.size();
@@ -2321,10 +2325,8 @@ int isspa_get_point_fields(isspa_engine *e, float *xyz, float *w, int *n, float 
     int rc = guard(e);
     if (rc) return rc;
     return run_guarded([&] {
-        if (!e->raw_e) {
-            e->raw_e = e->alloc<float4>(e->n_points);
-            e->raw_e0 = e->alloc<float4>(e->n_points);
-        }
+        e->alloc_once(e->raw_e, e->n_points);
+        e->alloc_once(e->raw_e0, e->n_points);
         launch_field(e->field_args(), e->field_split, true, e->stream);
         ck(cudaGetLastError());
         std::vector<float4> a(e->n_points), b(e->n_points), c(e->n_points);
