@@ -998,7 +998,7 @@ __global__ void __launch_bounds__(FieldShape<S>::kThreads, 1024 / FieldShape<S>:
                 }
         }
         __syncthreads();
-        if (!s_ok) return;
+        if (!s_ok) return leave_unchanged(m.lf, threadIdx.x, kT);
         for (int i = threadIdx.x; i < m.lf.n_atoms; i += kT) {
             // the other copies of the accumulator: read all at once, cleared
             long long extra[3] = {0, 0, 0}, c[kMergedCopies - 1][3];
@@ -1098,9 +1098,9 @@ __global__ void __launch_bounds__(kFieldThreads, 4) step_kernel(StepArgs a) {
     }
     bonded_terms(a.integ.bonded);
     restraint_coms(a.integ);
-    if (!grid_barrier(a.integ.bar, a.integ.lf.status)) return;
+    if (!grid_barrier(a.integ.bar, a.integ.lf.status)) return leave_atoms_unchanged(a.integ);
     for (int t = blockIdx.x; t < a.force.n_items; t += gridDim.x) force_item<true, 1>(a.force, t);
-    if (!grid_barrier(a.integ.bar, a.integ.lf.status)) return;
+    if (!grid_barrier(a.integ.bar, a.integ.lf.status)) return leave_atoms_unchanged(a.integ);
     integrate_atoms(a.integ, step);
 }
 

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(kUsThreads) integrator_kernel(IntegratorArgs a
     const uint32_t step = *a.lf.step_ptr;
     restraint_coms(a);
     bonded_terms(a.bonded);
-    if (!grid_barrier(a.bar, a.lf.status)) return;
+    if (!grid_barrier(a.bar, a.lf.status)) return leave_atoms_unchanged(a);
     integrate_atoms(a, step);
 }
 

@@ -532,6 +532,15 @@ __device__ __forceinline__ void leapfrog_atom(const LeapfrogArgs &a, int i, uint
     leapfrog_finish(a, i, leapfrog_prepare(a, i, step), extra);
 }
 
+// The atoms of a step that gives up: host buffers asked for get the state as it stays.
+__device__ __forceinline__ void leave_unchanged(const LeapfrogArgs &a, long long first, long long stride) {
+    for (long long i = first; i < a.n_atoms; i += stride) {
+        if (a.host_pos) a.host_pos[i] = a.pos[i];
+        if (a.host_vel) a.host_vel[i] = a.vel[i];
+        if (a.host_force) a.host_force[i] = a.force_out[i];
+    }
+}
+
 __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int *p) {
     unsigned int v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -601,6 +610,9 @@ __device__ __forceinline__ void bonded_terms(const BondedArgs &b) {
     const FixAdd add{b.facc, b.status};
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n_terms; t += stride)
         bonded_term(b, t, add);
+}
+__device__ __forceinline__ void leave_atoms_unchanged(const IntegratorArgs &a) {
+    leave_unchanged(a.lf, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
 // After the grid barrier: every atom adds its restraint force from its
 // window's COM axis (the umbrella kernel's fixed-point values) and is
