@@ -116,8 +116,8 @@ typedef struct isspa_engine_options {
                               all force_chunk items (about two waves of them); 0 => none */
     int field_vote;      /* 1: the field pass walks its atoms in groups of four with one
                             warp vote on "any inside rmax" per group (same results);
-                            0 => by the split and the box, per-pair branches once
-                            autotuning has measured them faster */
+                            0: per-pair branches; < 0 (the default) => by the split and
+                            the box, until autotuning keeps the faster */
     int force_vote;      /* 0 or 1, reported back; the force pass (one atom per thread)
                             takes its points in groups of four with one warp vote per
                             group either way */

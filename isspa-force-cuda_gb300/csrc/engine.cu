@@ -366,9 +366,10 @@ struct isspa_engine {
     }
 
     // ---------------------------------------------------------------- args
+    bool field_voted() const { return field_vote || (field_auto && default_vote(field_split, box_over_rmax)); }
     FieldArgs field_args() const {
         FieldArgs a{};
-        a.vote = field_vote || (field_auto && default_vote(field_split, box_over_rmax));
+        a.vote = field_voted();
         a.tma = field_tma;
         a.pos = pos;
         a.atype = atype;
@@ -1152,7 +1153,7 @@ void build(isspa_engine &E, const std::vector<isspa_host_system> &ws) {
     if (S != 1 && S != 2 && S != 4 && S != 8 && S != 16) S = E.default_field_split();
     E.set_field_split(S);
     E.field_vote = E.opt.field_vote == 1 ? 1 : 0;
-    E.field_auto = E.opt.field_vote == 0;
+    E.field_auto = E.opt.field_vote < 0;
     float box = 0.0f, rmax = 0.0f;
     for (const WinDev &d : E.win_h) box = std::max(box, d.box);
     for (float x : f0.rmax) rmax = std::max(rmax, x);
@@ -1407,6 +1408,7 @@ void isspa_default_options(isspa_engine_options *o) {
     o->isspa_terms = 7;
     o->nonbond_terms = 7;
     o->use_graph = 1;
+    o->field_vote = -1;
 }
 
 int isspa_engine_create(const isspa_system_desc *windows, int n_windows, const isspa_engine_options *opt,
@@ -1488,7 +1490,7 @@ int isspa_engine_shapes(const isspa_engine *e, int shape[ISSPA_SHAPE_COUNT]) {
     shape[6] = e->n_sms;
     shape[7] = e->force_apt;
     shape[8] = e->force_tail;
-    shape[9] = e->field_vote;
+    shape[9] = e->field_voted() ? 1 : 0;
     shape[10] = e->force_apt == 1 ? e->force_vote : 0;
     shape[11] = e->integrator;
     shape[12] = e->field_tma;

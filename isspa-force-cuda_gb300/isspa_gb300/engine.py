@@ -24,7 +24,7 @@ class Engine:
     def __init__(self, windows: "System | Sequence[System]", isspa_terms: int = 7,
                  nonbond_terms: int = 7, use_graph: bool = True, field_split: int = 0,
                  force_chunk: int = 0, mem_cap: int = 0, force_atoms_per_thread: int = 0,
-                 force_tail_chunk: int = 0, field_vote: int = 0, force_vote: int = 0, integrator: int = 0,
+                 force_tail_chunk: int = 0, field_vote: int = -1, force_vote: int = 0, integrator: int = 0,
                  nonbond_chunk: int = 0, field_tma: int = 0, nonbond_cutoff: float = 0.0,
                  nonbond_skin: float = 0.0, nonbond_list_max: int = 0, step_pdl: int = 0,
                  isspa_fused: int = 0, force_overlap: int = 0):
