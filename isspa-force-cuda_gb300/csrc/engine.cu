@@ -719,6 +719,10 @@ struct isspa_engine {
         launch_umbrella(umbrella_args(), s);
         launch_leapfrog(leapfrog_args(), s);
     }
+    // Programmatic launches of the step's chain; merged steps also unasked:
+    // autotuning times graphs of one step, where they do not show (back to back 44 /
+    // ADI2 / 264 atoms 7.4 / 9.5 / 20.8 us, 8.9 / 10.6 / 22.5 without)
+    bool steps_pdl() const { return step_pdl == 1 || (opt.step_pdl == 0 && merged()); }
     // Which kernels a step launches (the wrappers skip empty work lists).
     bool launches(int k) const {
         if (merged()) return k == ISSPA_K_STEP;
@@ -748,11 +752,8 @@ struct isspa_engine {
             if (timed && launches(k)) ck(cudaEventRecordWithFlags(kev[2 * k + end], s, cudaEventRecordExternal));
         };
         // programmatic launches for the field -> force -> leapfrog chain (not
-        // in the event-instrumented copy, whose event nodes sit between them);
-        // merged steps unasked: autotuning times graphs of one step, where they
-        // do not show (back to back 44 / ADI2 / 264 atoms 7.4 / 9.5 / 20.8 us, 8.9 /
-        // 10.6 / 22.5 without)
-        PdlScope pdl((step_pdl == 1 || (opt.step_pdl == 0 && merged())) && !timed && integrator != 3);
+        // in the event-instrumented copy, whose event nodes sit between them)
+        PdlScope pdl(steps_pdl() && !timed && integrator != 3);
         if (integrator == 3) {  // the whole step in one cooperative kernel
             mark(ISSPA_K_STEP, 0, stream);
             if (n_atoms > 0) ck(launch_step(step_args(), step_grid(), stream));
@@ -1496,7 +1497,7 @@ int isspa_engine_shapes(const isspa_engine *e, int shape[ISSPA_SHAPE_COUNT]) {
     shape[12] = e->field_tma;
     shape[13] = e->cutoff ? e->nbl_row_cap : 0;
     shape[14] = e->cutoff ? e->nbl_cells : 0;
-    shape[15] = e->step_pdl;
+    shape[15] = e->steps_pdl() ? 1 : 0;
     shape[16] = e->fused() ? 1 : 0;
     shape[17] = e->overlap() ? 1 : 0;
     return ISSPA_OK;
@@ -1959,6 +1960,14 @@ int isspa_autotune(isspa_engine *e, int reps, int shape[ISSPA_SHAPE_COUNT]) {
                 e->isspa_fused = c.fused;
                 e->force_overlap = c.ov;
             };
+            // (a merged step launches programmatically either way)
+            if (e->opt.step_pdl == 0)
+                cand.erase(std::remove_if(cand.begin(), cand.end(),
+                                          [&](const Cand &c) {
+                                              apply(c);
+                                              return c.pdl == 0 && e->merged();
+                                          }),
+                           cand.end());
             std::vector<float> t(cand.size(), 1e30f);
             int rounds = 3;
             for (int round = 0; round < rounds; ++round)

@@ -39,3 +39,20 @@ def test_tuned_engine():
     eng = ig.Engine(s)
     shapes = eng.autotune(reps=1)
     assert _replay(s, shapes) == shapes
+
+
+@pytest.mark.parametrize("option, reported", [(0, 1), (1, 1), (2, 0)])
+def test_merged_step_pdl(option, reported):
+    """Merged steps launch as programmatic dependents unless told not to."""
+    s = ig.synth.make_system(2, 22, 36.0, 5, seed=3, ff=ig.synth.forcefield(n_mc=5))
+    shapes = ig.Engine(s, isspa_fused=1, field_split=8, integrator=1, step_pdl=option).shapes()
+    assert shapes["step_pdl"] == reported
+    assert _replay(s, shapes) == shapes
+
+
+def test_tuned_merged_engine():
+    s = ig.synth.make_system(2, 22, 36.0, 5, seed=3, ff=ig.synth.forcefield(n_mc=5))
+    shapes = ig.Engine(s, integrator=1, isspa_fused=1).autotune(reps=1)
+    assert shapes["isspa_fused"] == 1
+    assert shapes["step_pdl"] == 1 or shapes["field_split"] == 4
+    assert _replay(s, shapes) == shapes
