@@ -55,6 +55,8 @@ __device__ __forceinline__ DF df_addf(DF a, float b) {
     const DF s = two_sum(a.hi, b);
     return fast_two_sum(s.hi, __fadd_rn(s.lo, a.lo));
 }
+// a times a power of two
+__device__ __forceinline__ DF df_scale(DF a, float p) { return DF{__fmul_rn(a.hi, p), __fmul_rn(a.lo, p)}; }
 // a b + c
 __device__ __forceinline__ DF df_fma(DF a, DF b, DF c) { return df_add(df_mul(a, b), c); }
 // x^2 + y^2 + z^2 (the compensated dot product of Ogita, Rump & Oishi 2005)

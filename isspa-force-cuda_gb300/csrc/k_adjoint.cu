@@ -178,6 +178,22 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_points_kernel(AdjointArgs
     if (valid) a.lam[p] = df_double(lam);
 }
 
+// A density factor v0 + f (v1 - v0) as m 2^e: e = 0 and the FP32 words as they are
+// within 2^+-32, else from FP64 (tables have zeros in the core, seldom values that
+// small).  The density product has an exponent of its own, so that neither it nor
+// its low word is lost where FP64 would hold them.
+constexpr float kFactorLow = 1.0f / 4294967296.0f, kFactorHigh = 4294967296.0f;
+__device__ __forceinline__ bool factor_range(float v) { return fabsf(v) >= kFactorLow && fabsf(v) <= kFactorHigh; }
+__device__ __forceinline__ DF density_factor(float v0, float v1, DF f, int &e) {
+    DF g = df_lerp(v0, v1, f);
+    e = 0;
+    if (!factor_range(g.hi) && (v0 != 0.0f || v1 != 0.0f)) {
+        const double fd = df_double(f);
+        g = df_from(frexp((double)v0 * (1.0 - fd) + (double)v1 * fd, &e));
+    }
+    return g;
+}
+
 // dJ/dT_g of one point per thread, in two sweeps over the point's in-range
 // atoms: the density product, then every factor's share lambda/n * prod / g.
 // The window's atoms are tested once in FP32 (once per sweep for windows beyond
@@ -207,7 +223,8 @@ __global__ void __launch_bounds__(kAdjThreads, 10) adjoint_density_kernel(Adjoin
     const DF g_inv = df_div(DF{1.f, 0.f}, DF{a.g_dr, 0.f});
     int zeros = 0;
     bool forced = false;
-    DF prod{1.0f, 0.0f};
+    DF prod{1.0f, 0.0f};  // of the nonzero factors, times 2^prod_e
+    int prod_e = 0;
     double *dg = a.dJ_dg + (long long)w * a.n_gtab;
     const int N = W.n_atoms, t = threadIdx.x;
     for (int pass = 0; pass < 2; ++pass) {
@@ -249,14 +266,29 @@ __global__ void __launch_bounds__(kAdjThreads, 10) adjoint_density_kernel(Adjoin
                     const int gi = __float_as_int(xj.w) + bin;
                     const bool next = gi + 1 < a.n_gtab;
                     const float g0 = __ldg(a.g_table + gi), g1 = next ? __ldg(a.g_table + gi + 1) : 0.0f;
-                    const DF g = df_lerp(g0, g1, fr);
+                    int ge;
+                    const DF g = density_factor(g0, g1, fr, ge);
                     if (pass == 0) {
-                        if (g.hi == 0.0f) ++zeros;
-                        else prod = df_mul(prod, g);
+                        if (g.hi == 0.0f) {
+                            ++zeros;
+                        } else {
+                            prod = df_mul(prod, g);
+                            prod_e += ge;
+                            if (!factor_range(prod.hi)) {
+                                const bool low = fabsf(prod.hi) < 1.0f;
+                                prod = df_scale(prod, low ? kFactorHigh : kFactorLow);
+                                prod_e += low ? -32 : 32;
+                            }
+                        }
                     } else if (!forced && (zeros == 0 || (zeros == 1 && g.hi == 0.0f))) {
                         // (of zero factors only a single one's own share survives)
                         const DF d = df_mul(dJdw, zeros ? prod : df_div(prod, g));
-                        if (d.hi != 0.0f) {
+                        const int de = zeros ? prod_e : prod_e - ge;
+                        if (de != 0) {
+                            const double v = scalbn(df_double(d), de), vf = v * df_double(fr);
+                            atomicAdd(dg + gi, v - vf);
+                            if (next) atomicAdd(dg + gi + 1, vf);
+                        } else if (d.hi != 0.0f) {
                             const DF df = df_mul(d, fr);
                             atomicAdd(dg + gi, df_sum(df_add(d, df_neg(df))));
                             if (next) atomicAdd(dg + gi + 1, df_sum(df));
