@@ -977,8 +977,8 @@ __global__ void __launch_bounds__(FieldShape<S>::kThreads, 1024 / FieldShape<S>:
     MergedSmem<S> &sm = *reinterpret_cast<MergedSmem<S> *>(s_dyn);
     int b = blockIdx.x;
     if (b == 0) {
-        // the integrator: everything but the force is ready when the last of
-        // the other blocks has added its share
+        // the integrator, an atom per thread (launch_merged_step): everything but
+        // the force is ready when the last of the other blocks has added its share
         __shared__ int s_ok;
         pdl_wait();
         pdl_trigger();
@@ -999,7 +999,8 @@ __global__ void __launch_bounds__(FieldShape<S>::kThreads, 1024 / FieldShape<S>:
         }
         __syncthreads();
         if (!s_ok) return leave_unchanged(m.lf, threadIdx.x, kT);
-        for (int i = threadIdx.x; i < m.lf.n_atoms; i += kT) {
+        if (threadIdx.x < m.lf.n_atoms) {
+            const int i = threadIdx.x;
             // the other copies of the accumulator: read all at once, cleared
             long long extra[3] = {0, 0, 0}, c[kMergedCopies - 1][3];
 #pragma unroll
@@ -1014,7 +1015,7 @@ __global__ void __launch_bounds__(FieldShape<S>::kThreads, 1024 / FieldShape<S>:
                     extra[k] += c[r][k];
                     if (r < m.n_copies - 1) m.copies[3 * ((long long)r * m.lf.n_atoms + i) + k] = 0ull;
                 }
-            leapfrog_finish(m.lf, i, i == threadIdx.x ? first : leapfrog_prepare(m.lf, i, step), extra);
+            leapfrog_finish(m.lf, i, first, extra);
         }
         if (threadIdx.x == 0) {  // every other block has read the step counter
             *m.lf.step_ptr = step + 1u;
@@ -1228,6 +1229,7 @@ cudaError_t merged_go(const MergedArgs &m, cudaStream_t s, bool prepare) {
 }  // namespace
 cudaError_t launch_merged_step(const MergedArgs &m, int split, cudaStream_t s, bool prepare) {
     if (m.lf.n_atoms <= 0) return cudaSuccess;
+    if ((split != 8 && split != 16) || m.lf.n_atoms > merged_threads(split)) return cudaErrorInvalidValue;
     const bool all = m.nonbond.terms == 7;
     if (split == 16) return all ? merged_go<16, true>(m, s, prepare) : merged_go<16, false>(m, s, prepare);
     return all ? merged_go<8, true>(m, s, prepare) : merged_go<8, false>(m, s, prepare);

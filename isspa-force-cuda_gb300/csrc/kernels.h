@@ -332,8 +332,9 @@ void launch_force(const ForceArgs &a, cudaStream_t s);
 // atom of its window right after their fields are known.
 bool field_force_fusable(int split);
 void launch_field_force(const FieldArgs &f, const ForceArgs &g, int split, cudaStream_t s);
-// The whole step in one launch (field split 4, 8 or 16; blocks of 32 threads per
-// split): its nonbond items hold up to merged_nonbond_partners() partners.
+// The whole step in one launch (field split 8 or 16; blocks of 32 threads per
+// split, and at most as many atoms): its nonbond items hold up to
+// merged_nonbond_partners() partners.
 constexpr int kMergedMaxLjTypes = 32;
 int merged_nonbond_partners(int split);
 int merged_threads(int split);
