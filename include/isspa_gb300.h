@@ -238,8 +238,8 @@ int isspa_engine_info(const isspa_engine *e, int *n_windows, int *n_atoms_total,
  * item, [3] force work items, [4] nonbond work items, [5] nonbond partners per
  * item, [6] SM count used for the choice, [7] receiving atoms per force
  * thread, [8] points per force work item of the short items listed last (0:
- * none), [9] 1 when the field pass walks its atoms in warp-voted groups,
- * [10] 1 when the force pass takes its points in warp-voted groups, [11] the
+ * none), [9] 1 when the field pass walks its atoms in warp-voted groups (by
+ * option, rule or autotuning), [10] the option force_vote as given, [11] the
  * step integrator (1 separate kernels, 2 fused, 3 single-kernel step; see isspa_engine_options),
  * [12] 1 when the field pass stages its atoms by bulk copies (TMA), [13] in
  * cutoff mode the partners a neighbour-list row holds (0 otherwise), [14] in
@@ -253,10 +253,8 @@ int isspa_engine_shapes(const isspa_engine *e, int shape[ISSPA_SHAPE_COUNT]);
  * loops, atoms staged by loads or by bulk copies) and, with one receiving atom
  * per force thread, a set of force-pass chunk lengths (those filling 1..12
  * whole waves of resident blocks, and powers of two; and long chunks followed
- * by about two waves of short ones; then the voted force loop on the chosen
- * list) on this engine's own
- * workload with CUDA events (reps launches each), keeps the fastest of each
- * and reports the result as isspa_engine_shapes does.  When the options leave
+ * by about two waves of short ones) on this engine's own workload with CUDA
+ * events (reps launches each), keeps the fastest of each and reports the result as isspa_engine_shapes does.  When the options leave
  * the integrator, step_pdl, isspa_fused or force_overlap open (0), it then
  * times single-step graph replays of the open choices (separate kernels, fused
  * integrator, single-kernel step; with and without programmatic launches;
@@ -304,7 +302,9 @@ int isspa_time_steps_detailed(isspa_engine *e, int nsteps, size_t flush_bytes, d
 int isspa_host_alloc(size_t bytes, void **out);
 void isspa_host_free(void *p);
 int isspa_synchronize(isspa_engine *e);
-/* Sticky device status word (0 if nothing tripped); clears it when reset != 0. */
+/* Sticky device status word (0 if nothing tripped); clears it when reset != 0,
+ * and with it, after ISSPA_ERR_TIMEOUT, the words of the waits that gave up and
+ * the force accumulator (the forces of steps that did not integrate). */
 int isspa_device_status(isspa_engine *e, int reset);
 /* Cutoff mode (no counterpart on the reference's live path; its dead
  * neighborlist_cuda.cu:11-137 / cell_list_cuda.cu:13-35 are the closest):

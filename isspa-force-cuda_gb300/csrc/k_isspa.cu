@@ -251,9 +251,8 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, F
             // attempts at every point at once and the first accepted one
             // counts (the points of one warp's sequential attempts, bit for
             // bit), instead of one warp drawing alone for the five or six
-            // attempts of its unluckiest lane while the others wait (1100
-            // atoms, S = 8: barrier stalls 1.9 -> 0.7 warps per issue; 44 atoms,
-            // S = 16, with the Langevin change: 11.4 -> 10.5 us per launch)
+            // attempts of its unluckiest lane while the others wait (when
+            // taken, 1100 atoms, S = 8: barrier stalls 1.9 -> 0.7 warps per issue)
             bool open = true;
             for (uint32_t att = 0;; att += S) {
                 float x, y, z;
@@ -402,48 +401,48 @@ __device__ __forceinline__ void field_tile(const FieldArgs &a, int tile_index, F
         bool inside = true;
         for (int q = sp + S * lane; q < jn; q += 32 * S) inside = inside && in_box(s_atom[TMA ? buf : 0][q], L);
         auto round = [&](auto toward) {
-        int k = sp;
-        // Groups of kG staged atoms: one warp vote tells whether any lane has
-        // any of them inside rmax.  When none does, their out-of-range Coulomb
-        // terms are summed without per-pair branches; the accumulators see the
-        // same operations in the same order either way.  It pays where few
-        // groups have an atom in range and where few warps share a tile (8800
-        // atoms, S = 1, 5496 against 6083 us per launch; 1100 atoms, S = 4, 87.8
-        // against 92.6), and costs registers where neither holds (1100 atoms,
-        // S = 16, 97.3 against 94.5): default_vote, or the autotuner's choice.
-        constexpr int kG = 4;
-        for (; VOTE && k + (kG - 1) * S < jn; k += kG * S) {
-            float rx[kG], ry[kG], rz[kG], c[kG];
-            bool any = false;
+            int k = sp;
+            // Groups of kG staged atoms: one warp vote tells whether any lane has
+            // any of them inside rmax.  When none does, their out-of-range Coulomb
+            // terms are summed without per-pair branches; the accumulators see the
+            // same operations in the same order either way.  It pays where few
+            // groups have an atom in range and where few warps share a tile (8800
+            // atoms, S = 1, 5496 against 6083 us per launch; 1100 atoms, S = 4, 87.8
+            // against 92.6), and costs registers where neither holds (1100 atoms,
+            // S = 16, 97.3 against 94.5): default_vote, or the autotuner's choice.
+            constexpr int kG = 4;
+            for (; VOTE && k + (kG - 1) * S < jn; k += kG * S) {
+                float rx[kG], ry[kG], rz[kG], c[kG];
+                bool any = false;
 #pragma unroll
-            for (int u = 0; u < kG; ++u) any = geom(toward, k + u * S, rx[u], ry[u], rz[u], c[u]) || any;
-            if (__any_sync(0xffffffffu, any)) {
+                for (int u = 0; u < kG; ++u) any = geom(toward, k + u * S, rx[u], ry[u], rz[u], c[u]) || any;
+                if (__any_sync(0xffffffffu, any)) {
 #pragma unroll
-                for (int u = 0; u < kG; ++u) accum(k + u * S, rx[u], ry[u], rz[u], c[u]);
-            } else {
+                    for (int u = 0; u < kG; ++u) accum(k + u * S, rx[u], ry[u], rz[u], c[u]);
+                } else {
 #pragma unroll
-                for (int u = 0; u < kG; ++u) {
-                    fx = fmaf(-c[u], rx[u], fx);
-                    fy = fmaf(-c[u], ry[u], fy);
-                    fz = fmaf(-c[u], rz[u], fz);
+                    for (int u = 0; u < kG; ++u) {
+                        fx = fmaf(-c[u], rx[u], fx);
+                        fy = fmaf(-c[u], ry[u], fy);
+                        fz = fmaf(-c[u], rz[u], fz);
+                    }
                 }
             }
-        }
-        if (VOTE) {
+            if (VOTE) {
 #pragma unroll 1
-            for (; k < jn; k += S) {  // at most kG - 1 atoms
-                float rx, ry, rz, c;
-                geom(toward, k, rx, ry, rz, c);
-                accum(k, rx, ry, rz, c);
-            }
-        } else {
+                for (; k < jn; k += S) {  // at most kG - 1 atoms
+                    float rx, ry, rz, c;
+                    geom(toward, k, rx, ry, rz, c);
+                    accum(k, rx, ry, rz, c);
+                }
+            } else {
 #pragma unroll 4
-            for (; k < jn; k += S) {
-                float rx, ry, rz, c;
-                geom(toward, k, rx, ry, rz, c);
-                accum(k, rx, ry, rz, c);
+                for (; k < jn; k += S) {
+                    float rx, ry, rz, c;
+                    geom(toward, k, rx, ry, rz, c);
+                    accum(k, rx, ry, rz, c);
+                }
             }
-        }
         };
         if (__all_sync(0xffffffffu, inside)) round(std::true_type{});
         else round(std::false_type{});
@@ -708,43 +707,43 @@ __device__ __forceinline__ void force_item(const ForceArgs &a, int item_index) {
                                                   lx[u], ly[u], lz[u]);
         };
         auto stage = [&](auto toward) {
-        constexpr bool T = decltype(toward)::value;
-        int k = 0;
-        if (A == 1) {
-            for (; k + 3 < pn; k += 4) {
-                float rx[4], ry[4], rz[4], d2[4];
-                bool any = false;
+            constexpr bool T = decltype(toward)::value;
+            int k = 0;
+            if (A == 1) {
+                for (; k + 3 < pn; k += 4) {
+                    float rx[4], ry[4], rz[4], d2[4];
+                    bool any = false;
 #pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const float4 P = s_p[k + v].q[0];
-                    const float4 sd = T ? s_side[k + v] : P;
-                    rx[v] = image<T>(P.x - xi[0].x, sd.x, L, h);
-                    ry[v] = image<T>(P.y - xi[0].y, sd.y, L, h);
-                    rz[v] = image<T>(P.z - xi[0].z, sd.z, L, h);
-                    d2[v] = dist2f(rx[v], ry[v], rz[v]);
-                    any = any || d2[v] <= rm2[0];
-                }
-                if (__any_sync(0xffffffffu, any)) {
+                    for (int v = 0; v < 4; ++v) {
+                        const float4 P = s_p[k + v].q[0];
+                        const float4 sd = T ? s_side[k + v] : P;
+                        rx[v] = image<T>(P.x - xi[0].x, sd.x, L, h);
+                        ry[v] = image<T>(P.y - xi[0].y, sd.y, L, h);
+                        rz[v] = image<T>(P.z - xi[0].z, sd.z, L, h);
+                        d2[v] = dist2f(rx[v], ry[v], rz[v]);
+                        any = any || d2[v] <= rm2[0];
+                    }
+                    if (__any_sync(0xffffffffu, any)) {
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) pair(k + v, 0, rx[v], ry[v], rz[v], d2[v], std::false_type{});
-                } else {
+                        for (int v = 0; v < 4; ++v) pair(k + v, 0, rx[v], ry[v], rz[v], d2[v], std::false_type{});
+                    } else {
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) pair(k + v, 0, rx[v], ry[v], rz[v], d2[v], std::true_type{});
+                        for (int v = 0; v < 4; ++v) pair(k + v, 0, rx[v], ry[v], rz[v], d2[v], std::true_type{});
+                    }
                 }
             }
-        }
 #pragma unroll 4
-        for (; k < pn; ++k) {
-            const float4 P = s_p[k].q[0];
-            const float4 sd = T ? s_side[k] : P;
+            for (; k < pn; ++k) {
+                const float4 P = s_p[k].q[0];
+                const float4 sd = T ? s_side[k] : P;
 #pragma unroll
-            for (int u = 0; u < A; ++u) {
-                const float rx = image<T>(P.x - xi[u].x, sd.x, L, h);
-                const float ry = image<T>(P.y - xi[u].y, sd.y, L, h);
-                const float rz = image<T>(P.z - xi[u].z, sd.z, L, h);
-                pair(k, u, rx, ry, rz, dist2f(rx, ry, rz), std::false_type{});
+                for (int u = 0; u < A; ++u) {
+                    const float rx = image<T>(P.x - xi[u].x, sd.x, L, h);
+                    const float ry = image<T>(P.y - xi[u].y, sd.y, L, h);
+                    const float rz = image<T>(P.z - xi[u].z, sd.z, L, h);
+                    pair(k, u, rx, ry, rz, dist2f(rx, ry, rz), std::false_type{});
+                }
             }
-        }
         };
         if (toward) stage(std::true_type{});
         else stage(std::false_type{});

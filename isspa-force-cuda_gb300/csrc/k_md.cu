@@ -1,11 +1,11 @@
 // k_md.cu -- pair, bonded, umbrella and integrator kernels for sm_103a.
 //
 //  nonbond:  all-pairs LJ + Coulomb + IS-SPA long-range dielectric correction
-//            (reference src/nonbond_force_cuda.cu:31-174).  One thread per
-//            receiving atom, partner atoms streamed through shared memory,
-//            exclusions from a per-atom sorted list walked with a cursor (the
-//            reference copies the whole list into shared memory per block and
-//            fails once it exceeds 48 KB).
+//            (reference src/nonbond_force_cuda.cu:31-174).  32 receiving atoms
+//            per block, one per lane of four warps that take groups of 32 staged
+//            partners in turn; exclusions as a 32-bit mask per group from a
+//            per-atom sorted list (the reference copies the whole list into
+//            shared memory per block and fails once it exceeds 48 KB).
 //  bonded:   bonds, angles, dihedrals with scaled 1-4 (bond_force_cuda.cu:
 //            15-53, angle_force_cuda.cu:12-66, dih_force_cuda.cu:13-136) in one
 //            launch over the concatenated term lists.

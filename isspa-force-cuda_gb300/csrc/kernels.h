@@ -390,7 +390,11 @@ int field_blocks_per_sm(int split);
 // Us per launch at S = 1 / 2 / 4 / 8 / 16: 8800 atoms (nMC 100) 5496 / 5867 / 6223 /
 // 6402 / 6850, 4400 930 / 832 / 870 / 890 / 962, windows of 44 to 1100 atoms 292 /
 // 299 / 312 / 326 / 387, 1100 atoms 107 / 91 / 88 / 87 / 95, 741 79 / 52 / 42 / 43 /
-// 43, 264 54 / 33 / 24 / 17 / 16.5.  tiles(S): a split's number of tiles.
+// 43, 264 54 / 33 / 24 / 17 / 16.5.  kCost follows the rows of a full chip, except
+// that 16 stands above its 1.25 (with that, 1100 atoms would take 16, 95 against 87 us)
+// and 2 above its 1.02 to 1.07 (below 1.06 a 16 384-atom window would take 2).  The
+// rule misses 4400 atoms: their 1719 tiles of a split of 1 fill 94 % of one wave, and
+// it takes 1 where 2 measured 832 against 930.  tiles(S): a split's number of tiles.
 template <class Tiles>
 int default_split(int sms, const Tiles &tiles) {
     auto whole = [](long long units, long long slots) {  // filled share of the rounds
