@@ -178,20 +178,16 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_points_kernel(AdjointArgs
     if (valid) a.lam[p] = df_double(lam);
 }
 
-// A density factor v0 + f (v1 - v0) as m 2^e: e = 0 and the FP32 words as they are
-// within 2^+-32, else from FP64 (tables have zeros in the core, seldom values that
-// small).  The density product has an exponent of its own, so that neither it nor
-// its low word is lost where FP64 would hold them.
-constexpr float kFactorLow = 1.0f / 4294967296.0f, kFactorHigh = 4294967296.0f;
-__device__ __forceinline__ bool factor_range(float v) { return fabsf(v) >= kFactorLow && fabsf(v) <= kFactorHigh; }
+// The density product is held as prod 2^prod_e with prod within 2^+-32, so that
+// neither it nor its low word is lost where FP64 would hold them; a factor v0 + f (v1
+// - v0) that leads out of that range is taken from FP64 as m 2^e (tables have zeros in
+// the core, seldom values that small: a factor 0 is the common case here).
+constexpr float kRange = 4294967296.0f;  // 2^32
+__device__ __forceinline__ bool in_range(float v) { return fabsf(v) >= 1.0f / kRange && fabsf(v) <= kRange; }
 __device__ __forceinline__ DF density_factor(float v0, float v1, DF f, int &e) {
-    DF g = df_lerp(v0, v1, f);
-    e = 0;
-    if (!factor_range(g.hi) && (v0 != 0.0f || v1 != 0.0f)) {
-        const double fd = df_double(f);
-        g = df_from(frexp((double)v0 * (1.0 - fd) + (double)v1 * fd, &e));
-    }
-    return g;
+    if (v0 == 0.0f && v1 == 0.0f) return DF{0.0f, 0.0f};
+    const double fd = df_double(f);
+    return df_from(frexp((double)v0 * (1.0 - fd) + (double)v1 * fd, &e));
 }
 
 // dJ/dT_g of one point per thread, in two sweeps over the point's in-range
@@ -266,22 +262,24 @@ __global__ void __launch_bounds__(kAdjThreads, 10) adjoint_density_kernel(Adjoin
                     const int gi = __float_as_int(xj.w) + bin;
                     const bool next = gi + 1 < a.n_gtab;
                     const float g0 = __ldg(a.g_table + gi), g1 = next ? __ldg(a.g_table + gi + 1) : 0.0f;
-                    int ge;
-                    const DF g = density_factor(g0, g1, fr, ge);
+                    DF g = df_lerp(g0, g1, fr);
+                    int ge = 0;
                     if (pass == 0) {
-                        if (g.hi == 0.0f) {
+                        const DF p = df_mul(prod, g);
+                        if (in_range(p.hi)) {
+                            prod = p;
+                        } else if ((g = density_factor(g0, g1, fr, ge)).hi == 0.0f) {
                             ++zeros;
                         } else {
                             prod = df_mul(prod, g);
-                            prod_e += ge;
-                            if (!factor_range(prod.hi)) {
-                                const bool low = fabsf(prod.hi) < 1.0f;
-                                prod = df_scale(prod, low ? kFactorHigh : kFactorLow);
-                                prod_e += low ? -32 : 32;
-                            }
+                            const int up = fabsf(prod.hi) < 1.0f / kRange ? 32 : 0;
+                            prod = df_scale(prod, up ? kRange : 1.0f);
+                            prod_e += ge - up;
                         }
-                    } else if (!forced && (zeros == 0 || (zeros == 1 && g.hi == 0.0f))) {
-                        // (of zero factors only a single one's own share survives)
+                    } else if (!forced) {
+                        // of zero factors only a single one's own share survives
+                        if (!in_range(g.hi)) g = density_factor(g0, g1, fr, ge);
+                        if (zeros > 1 || (zeros == 1 && g.hi != 0.0f)) continue;
                         const DF d = df_mul(dJdw, zeros ? prod : df_div(prod, g));
                         const int de = zeros ? prod_e : prod_e - ge;
                         if (de != 0) {
