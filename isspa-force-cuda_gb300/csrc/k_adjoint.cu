@@ -19,7 +19,8 @@
 // the sums.  16 windows x 550 atoms, nMC 50, per launch: points 6.76 ms in FP64,
 // 0.30 in double-float; density 12.0 ms, 2.4 with the double-float body, 0.91
 // once the warp reconverges after each lane's own atoms, 0.81 with one FP32 test
-// per atom and point, 0.82 with the product's exponent; pairs 0.88 ms with a thread per atom, 0.07 with a warp.
+// per atom and point, 0.82 with the product's exponent; pairs 0.88 ms with a thread
+// per atom, 0.07 with a warp.
 // The error against 64-bit references is the FP32 fields' and coordinates'
 // either way (6e-6 of dJ/dT_g at those sizes, before and after).
 #include <algorithm>
